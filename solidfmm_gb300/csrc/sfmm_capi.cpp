@@ -77,6 +77,14 @@ cudaError_t upload(void **dst, const std::vector<double> &v, Arith a)
     return cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
 }
 
+void free_fx(FxDevTables &t)
+{
+    void *ps[] = {t.W, t.H[0], t.H[1], t.H[2], t.woff, t.hoff};
+    for (void *p : ps)
+        if (p) cudaFree(p);
+    t = FxDevTables{};
+}
+
 void free_tables(DevTables &t)
 {
     void *ps[] = {t.W, t.ein_M, t.ein_L, t.eout_L, t.eout_M, t.H[0], t.H[1], t.H[2], t.Wq, t.W8, t.Wq8};
@@ -157,6 +165,51 @@ int ensure_tables(sfmm_context *c, Arith a)
 }
 
 
+// Tables of the 60-bit fixed-point kernel for G threads per translation
+// (orders up to 32), once per context.
+int ensure_fx(sfmm_context *c, int G)
+{
+    FxDevTables &t = c->fxt[G == 8];
+    if (t.ready) return SFMM_OK;
+    const int P = std::min(c->P, 32);
+    auto put = [](void **dst, const void *src, size_t bytes) {
+        cudaError_t e = cudaMalloc(dst, bytes);
+        if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+        return e;
+    };
+    cudaError_t e = cudaSuccess;
+    try {
+        const std::vector<double> *ev[4] = {&c->host.e_in_M, &c->host.e_in_L, &c->host.e_out_L, &c->host.e_out_M};
+        for (int k = 0; k < 4 && e == cudaSuccess; ++k) {
+            if (c->fx_edge[k]) continue;
+            const auto v = fx_edges(*ev[k], (size_t)P * (P + 1) / 2);
+            e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(int32_t));
+            if (e != cudaSuccess && c->fx_edge[k]) {
+                cudaFree(c->fx_edge[k]);
+                c->fx_edge[k] = nullptr;
+            }
+        }
+        const FxTables h = build_fx_tables(c->host, G, P);
+        t.wend.assign(P + 1, (int)(h.W.size() * sizeof(int32_t)));
+        for (int n = 0; n < P; ++n) t.wend[n] = h.woff[n] * 8;
+        t.hbytes = (int)(h.H[0].size() * sizeof(double));
+        if (e == cudaSuccess) e = put(&t.W, h.W.data(), h.W.size() * sizeof(int32_t));
+        for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k].data(), h.H[k].size() * sizeof(double));
+        if (e == cudaSuccess) e = put((void **)&t.woff, h.woff.data(), h.woff.size() * sizeof(int));
+        if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff.data(), h.hoff.size() * sizeof(int));
+    } catch (const std::bad_alloc &) {
+        free_fx(t);
+        return fail(c, SFMM_OOM, "operator tables");
+    }
+    if (e != cudaSuccess) {
+        free_fx(t);  // a partial set is retried from scratch on the next call
+        return cuda_fail(c, e, "table upload");
+    }
+    t.P = P;
+    t.ready = true;
+    return SFMM_OK;
+}
+
 int arith_of(sfmm_context *c, int precision, Arith *out)
 {
     if (precision == SFMM_PLAIN) {
@@ -193,14 +246,20 @@ Arith resolve_arith(Arith a, int op, int Pbound)
     return a;
 }
 
+// the device tables that a launch of this shape reads (setup_mtx held)
+static int ensure_shape_tables(sfmm_context *c, Arith a, const LaunchShape &s)
+{
+    return s.fx ? ensure_fx(c, s.G) : ensure_tables(c, a);
+}
+
 int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *shape)
 {
     a = resolve_arith(a, op, Pbound);
     if (Pbound < 1) Pbound = 1;
     std::lock_guard<std::mutex> lk(c->setup_mtx);
-    int st = ensure_tables(c, a);
-    if (st) return st;
     if (is_tc(a)) {  // one 128-thread CTA per SM, one translation per thread
+        int st = ensure_tables(c, a);
+        if (st) return st;
         if (shape) {
             *shape = LaunchShape{};
             shape->G = 1;
@@ -219,7 +278,7 @@ int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *sh
         return fail(c, SFMM_UNSUPPORTED, "order %d exceeds the GPU kernels' limit %d", Pbound, kMaxKernelOrder);
     if (a != Arith::F64 && Pbound > kMaxFloatOrder)
         return fail(c, SFMM_UNSUPPORTED, "order %d exceeds %d, the limit of FP32-range arithmetic", Pbound, kMaxFloatOrder);
-    return SFMM_OK;
+    return ensure_shape_tables(c, a, it->second);
 }
 
 void set_shape(sfmm_context *c, std::tuple<int, int, int> key, const LaunchShape *s)
@@ -256,7 +315,11 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
     LaunchShape s;
     int st = prepare_launch(c, op, a, Pbound, &s);
     if (st) return st;
-    if (shape && !is_tc(a)) s = *shape;
+    if (shape && !is_tc(a)) {
+        s = *shape;
+        std::lock_guard<std::mutex> lk(c->setup_mtx);
+        if ((st = ensure_shape_tables(c, a, s))) return st;
+    }
     KParams p{};
     p.op = op;
     p.P = Pbound;
@@ -292,18 +355,31 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
         c->launches++;
         return SFMM_OK;
     }
-    const DevTables &t = c->tab[(int)a];
-    // swap blocks padded for this launch's group size (4 or 8 threads per
-    // translation step 8 rows, one warp 32)
-    const bool w8 = s.G != 32 && c->d_woff8;
-    p.W = w8 ? t.W8 : t.W;
-    p.Wq = static_cast<const int *>(w8 ? t.Wq8 : t.Wq);
-    p.woff = w8 ? c->d_woff8 : c->d_woff;
-    p.hoff = c->d_hoff;
-    p.rowpad = c->host.pad;
-    p.ein = (op == SFMM_L2L) ? t.ein_L : t.ein_M;
-    p.eout = (op == SFMM_M2M) ? t.eout_M : t.eout_L;
-    p.H = t.H[op];
+    if (s.fx) {
+        const FxDevTables &t = c->fxt[s.G == 8];
+        p.W = t.W;
+        p.woff = t.woff;
+        p.hoff = t.hoff;
+        p.Ptab = t.P;
+        p.ein = c->fx_edge[op == SFMM_L2L ? 1 : 0];
+        p.eout = c->fx_edge[op == SFMM_M2M ? 3 : 2];
+        p.H = t.H[op];
+        p.wbytes = t.wend[Pbound];
+        p.hbytes = t.P == Pbound ? t.hbytes : 0;  // a smaller bound reads parts of every row
+    } else {
+        const DevTables &t = c->tab[(int)a];
+        // swap blocks padded for this launch's group size (4 or 8 threads per
+        // translation step 8 rows, one warp 32)
+        const bool w8 = s.G != 32 && c->d_woff8;
+        p.W = w8 ? t.W8 : t.W;
+        p.Wq = static_cast<const int *>(w8 ? t.Wq8 : t.Wq);
+        p.woff = w8 ? c->d_woff8 : c->d_woff;
+        p.hoff = c->d_hoff;
+        p.rowpad = c->host.pad;
+        p.ein = (op == SFMM_L2L) ? t.ein_L : t.ein_M;
+        p.eout = (op == SFMM_M2M) ? t.eout_M : t.eout_L;
+        p.H = t.H[op];
+    }
     p.spad = s.spad;
     p.TS = s.TS;
     long long tiles = wl ? wl->n : (n + s.TS - 1) / s.TS;
@@ -338,6 +414,20 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     int acc = (P + G - 1) / G;
     if (G == 4) acc = acc <= 2 ? 2 : (acc <= 4 ? 4 : (acc <= 6 ? 6 : 8));
     if (G == 32) acc = acc <= 2 ? 2 : 3;
+    // FP64 up to order 32 runs in 60-bit fixed point, rows in steps of G/2;
+    // four threads per translation only up to order 16 (more rows than their
+    // registers hold: above, a request for 4 runs 8)
+    s.fx = a == Arith::F64 && G != 32;
+    if (s.fx) {
+        if (P > 16 && G == 4) {
+            G = 8;
+            ts /= 2;
+            if (ts < 32 / G || ts % (32 / G)) return s;
+        }
+        if (G * ts > kFxThreads) return LaunchShape{};
+        acc = (P + G / 2 - 1) / (G / 2);
+        acc = G == 4 ? (acc <= 4 ? 4 : acc <= 6 ? 6 : 8) : (acc + 1) / 2 * 2;
+    }
     s.G = G;
     s.acc = acc;
     int scap = P * (P + 1) + 4;  // room for the swap loops' zero-coefficient reads past the last row
@@ -352,7 +442,7 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     s.spad = scap + ((want - scap) % mod + mod) % mod;
     s.TS = ts;
     s.threads = G * ts;
-    s.smem = (size_t)ts * s.spad * esize(a) + 5 * sizeof(uint32_t) * ts;
+    s.smem = (size_t)ts * s.spad * esize(a) + 5 * sizeof(uint32_t) * ts + (s.fx ? ts * sizeof(FxGeo) : 0);
     if (s.smem > 232448) return LaunchShape{};
     return s;
 }
@@ -361,12 +451,14 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
 // 8 from a sweep on GB300 (M2L, uniform orders 2..32, both group sizes): 8
 // threads pay off once the per-translation buffers limit the SM to a few
 // warps and the group's own arithmetic is cheap enough to leave latency
-// exposed (FP64 from order 24, FP32 from 17, both split modes from 14).
+// exposed (FP32 from 17, both split modes from 14).  FP64 (60-bit fixed point)
+// from 13, where four threads need more rows than fit the registers of a full
+// SM: M2L at P=12 189 M/s with 4 and 150 with 8, at P=13 89 and 125.
 int default_group(Arith a, int P)
 {
     if (P > 32) return 32;
     switch (a) {
-    case Arith::F64: return P >= 24 ? 8 : 4;
+    case Arith::F64: return P >= 13 ? 8 : 4;
     case Arith::F32: return P >= 17 ? 8 : 4;
     case Arith::FF: return P >= 14 ? 8 : 4;
     case Arith::FFQ: return P >= 14 ? 8 : 4;
@@ -384,27 +476,30 @@ LaunchShape best_shape(Arith a, int P, int G, bool small_tiles, int min_threads)
     // more threads per SM at high orders, but ran up to 40% slower on GB300
     // (split M2L P=22: 1 976 CTAs of 32 threads, instruction-fetch stalls and
     // a lower L1 hit rate for the tables); smaller CTAs when no larger tile
-    // fits, or when sfmm_tune measures them faster (split P=27: +6%).
-    for (int floor_threads : {min_threads, 32}) {
-        LaunchShape best;
-        long best_threads = 0;
+    // fits, or when sfmm_tune measures them faster (split P=27: +6%).  The
+    // 60-bit kernel also takes smaller ones where they hold an eighth more
+    // threads: M2L P=24 21.0 -> 25.4 M/s, P=32 7.3 -> 9.0, P=21 34.3 -> 36.2,
+    // while with fewer (P=20) or equal numbers four warps win (47.7 against 42.0).
+    LaunchShape best[2];
+    long most[2] = {0, 0};
+    for (int k = 0; k < 2; ++k)
         for (int ts = 256 / G; ts >= 32 / G; ts -= 32 / G) {
-            if (G * ts < floor_threads) break;
             LaunchShape s = translate_shape(a, P, G, ts);
-            if (!s.acc) continue;
+            if (!s.acc || s.threads < (k ? 32 : min_threads)) continue;
             s.blocks_per_sm = translate_blocks_per_sm(a, s);
-            long th = (long)s.blocks_per_sm * s.threads;
-            if (th > 0 && (th > best_threads || (small_tiles && th == best_threads))) {
-                best_threads = th;
-                best = s;
+            const long th = (long)s.blocks_per_sm * s.threads;
+            if (th > 0 && (th > most[k] || (small_tiles && th == most[k]))) {
+                most[k] = th;
+                best[k] = s;
             }
         }
-        if (best.acc) return best;
-    }
-    return LaunchShape{};
+    if (!best[0].acc || (best[0].fx && 8 * most[1] >= 9 * most[0])) return best[1];
+    return best[0];
 }
 
 cudaError_t launch_translate_64(const KParams &, const LaunchShape &, int, cudaStream_t);
+cudaError_t launch_translate_fx(const KParams &, const LaunchShape &, int, cudaStream_t);
+int occupancy_fx64(const LaunchShape &);
 cudaError_t launch_translate_32(const KParams &, const LaunchShape &, int, cudaStream_t);
 cudaError_t launch_translate_ff(const KParams &, const LaunchShape &, int, cudaStream_t);
 cudaError_t launch_translate_ffq(const KParams &, const LaunchShape &, int, cudaStream_t);
@@ -416,7 +511,7 @@ int occupancy_ffq(const LaunchShape &);
 cudaError_t launch_translate(Arith a, const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
 {
     switch (a) {
-    case Arith::F64: return launch_translate_64(p, s, grid, st);
+    case Arith::F64: return s.fx ? launch_translate_fx(p, s, grid, st) : launch_translate_64(p, s, grid, st);
     case Arith::F32: return launch_translate_32(p, s, grid, st);
     case Arith::FFQ: return launch_translate_ffq(p, s, grid, st);
     default: return launch_translate_ff(p, s, grid, st);
@@ -426,7 +521,7 @@ cudaError_t launch_translate(Arith a, const KParams &p, const LaunchShape &s, in
 int translate_blocks_per_sm(Arith a, const LaunchShape &s)
 {
     switch (a) {
-    case Arith::F64: return occupancy_64(s);
+    case Arith::F64: return s.fx ? occupancy_fx64(s) : occupancy_64(s);
     case Arith::F32: return occupancy_32(s);
     case Arith::FFQ: return occupancy_ffq(s);
     default: return occupancy_ff(s);
@@ -496,6 +591,9 @@ void sfmm_destroy(sfmm_context *c)
     cudaSetDevice(c->device);
     for (auto &t : c->tab) free_tables(t);
     for (auto &t : c->tc) tc_release(t);
+    for (auto &t : c->fxt) free_fx(t);
+    for (void *p : c->fx_edge)
+        if (p) cudaFree(p);
     for (int k = 0; k < 3; ++k) {
         c->d_src[k].release();
         c->d_dst[k].release();
@@ -577,6 +675,8 @@ int sfmm_set_group(sfmm_context *c, int precision, size_t order_bound, int group
             return fail(c, SFMM_INVALID_ARG, "no kernel runs %d threads per translation at order %d", group, Pb);
     }
     std::lock_guard<std::mutex> lk2(c->setup_mtx);
+    for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
+        if (s[op - SFMM_M2M].fx && (st = ensure_fx(c, group))) return st;  // before a capture may launch it
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
         c->shapes[std::make_tuple(op, (int)resolve_arith(a, op, Pb), Pb)] = s[op - SFMM_M2M];
     return SFMM_OK;

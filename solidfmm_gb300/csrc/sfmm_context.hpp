@@ -31,6 +31,18 @@ struct DevTables {
     bool ready = false;
 };
 
+// device tables of the 60-bit fixed-point kernel (sfmm_tables.hpp, FxTables),
+// one set per group size; the edge factors (e_in_M, e_in_L, e_out_L, e_out_M)
+// are shared by the sets
+struct FxDevTables {
+    void *W = nullptr, *H[3] = {nullptr, nullptr, nullptr};
+    int *woff = nullptr, *hoff = nullptr;
+    int P = 0;
+    std::vector<int> wend;  // bytes of the swap tables of degrees below an order bound
+    int hbytes = 0;         // of one operator's z matrices
+    bool ready = false;
+};
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -83,6 +95,8 @@ struct sfmm_context {
     cudaStream_t stream = nullptr;
     sfmm::HostTables host;
     sfmm::DevTables tab[sfmm::kNumArith];  // indexed by Arith (the tensor-core modes use tc[])
+    sfmm::FxDevTables fxt[2];  // 4 and 8 threads per translation
+    void *fx_edge[4] = {nullptr, nullptr, nullptr, nullptr};
     sfmm::TcDevTables *tc[3] = {nullptr, nullptr, nullptr};  // tensor-core operand images by format
     std::string err;
     std::atomic<uint64_t> launches{0};

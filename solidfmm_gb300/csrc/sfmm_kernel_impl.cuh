@@ -47,12 +47,26 @@ static int occupancy_inst(const LaunchShape &s)
 
 #define SFMM_FOR_SHAPES(X) \
     X(4, 2) X(4, 4) X(4, 6) X(4, 8) X(8, 1) X(8, 2) X(8, 3) X(8, 4) X(32, 2) X(32, 3)
+// 60-bit fixed point: rows in steps of G/2
+#ifndef SFMM_FOR_FX_SHAPES
+#define SFMM_FOR_FX_SHAPES(X) X(4, 4) X(4, 6) X(4, 8) X(8, 2) X(8, 4) X(8, 6) X(8, 8)
+#endif
+// which of the general shapes an arithmetic runs: the fixed-point float-float
+// variant none of one warp per translation, FP64 only those (the 60-bit kernel
+// runs the others)
+template <class A, bool FIX>
+constexpr bool runs_shape(int G, int acc)
+{
+    if (FIX) return G != 32;
+    if (std::is_same<A, double>::value) return G == 32;
+    return true;
+}
 
 template <class A, bool FIX = false>
 static cudaError_t launch_typed(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
 {
 #define X(G_, A_) \
-    if constexpr (!(FIX && G_ == 32))                                   \
+    if constexpr (runs_shape<A, FIX>(G_, A_))                           \
         if (s.G == G_ && s.acc == A_) return launch_inst<A, G_, A_, FIX>(p, s, grid, st);
     SFMM_FOR_SHAPES(X)
 #undef X
@@ -63,9 +77,54 @@ template <class A, bool FIX = false>
 static int occupancy_typed(const LaunchShape &s)
 {
 #define X(G_, A_) \
-    if constexpr (!(FIX && G_ == 32))              \
+    if constexpr (runs_shape<A, FIX>(G_, A_))      \
         if (s.G == G_ && s.acc == A_) return occupancy_inst<A, G_, A_, FIX>(s);
     SFMM_FOR_SHAPES(X)
+#undef X
+    return 0;
+}
+
+template <int G, int ACC>
+static cudaError_t launch_fx_inst(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
+{
+    clear_stale_error();
+    if (p.work) {
+        if (!p.in_hbm) return cudaErrorInvalidValue;  // work lists are a device-memory form
+        k_translate_fx<G, ACC, true, true><<<grid, s.threads, s.smem, st>>>(p);
+    } else if (p.in_hbm) {
+        k_translate_fx<G, ACC, true><<<grid, s.threads, s.smem, st>>>(p);
+    } else {
+        k_translate_fx<G, ACC, false><<<grid, s.threads, s.smem, st>>>(p);
+    }
+    return cudaGetLastError();
+}
+
+template <int G, int ACC>
+static int occupancy_fx_inst(const LaunchShape &s)
+{
+    auto kern = k_translate_fx<G, ACC>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    cudaFuncSetAttribute(k_translate_fx<G, ACC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    cudaFuncSetAttribute(k_translate_fx<G, ACC, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, s.threads, s.smem) != cudaSuccess) return 0;
+    return nb;
+}
+
+static inline cudaError_t launch_fx(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
+{
+#define X(G_, A_) \
+    if (s.G == G_ && s.acc == A_) return launch_fx_inst<G_, A_>(p, s, grid, st);
+    SFMM_FOR_FX_SHAPES(X)
+#undef X
+    return cudaErrorInvalidValue;
+}
+
+static inline int occupancy_fx(const LaunchShape &s)
+{
+#define X(G_, A_) \
+    if (s.G == G_ && s.acc == A_) return occupancy_fx_inst<G_, A_>(s);
+    SFMM_FOR_FX_SHAPES(X)
 #undef X
     return 0;
 }

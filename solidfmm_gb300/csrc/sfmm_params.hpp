@@ -5,6 +5,8 @@
 
 #include <vector_types.h>
 
+#include "sfmm_fx_layout.hpp"
+
 namespace sfmm {
 
 enum { OP_M2M = 0, OP_M2L = 1, OP_L2L = 2 };
@@ -12,6 +14,16 @@ enum { OP_M2M = 0, OP_M2L = 1, OP_L2L = 2 };
 // buffer slots per translation covered by the FP32-range kernels' table of
 // coefficient degrees (every order up to 28 with its padding)
 constexpr int kDegreeTableSize = 1024;
+
+// threads per CTA of the 60-bit fixed-point kernel, at most
+constexpr int kFxThreads = 128;
+
+// per-translation geometry of the 60-bit fixed-point kernel, in shared memory
+struct FxGeo {
+    long long ca, sa, cb, sb;  // Q60 cos / sin of alpha and beta
+    long long r, rinv;         // 60-bit mantissas of |shift| and 1/|shift|
+    int re, rinve;             // their exponents; kFxBad: not finite or zero
+};
 
 struct KParams {
     int op;
@@ -41,6 +53,7 @@ struct KParams {
     const void *ein;    // arith-typed forward edge factors (op dependent)
     const void *eout;   // arith-typed backward edge factors (op dependent)
     const void *H;      // arith-typed z matrices of this op
+    int wbytes, hbytes; // 60-bit kernel: bytes of W and H that this order bound reads
     int spad;           // buffer elements per translation
     int TS;             // translations per CTA tile
     void *scratch;      // global buffer (GBUF kernels)

@@ -4,6 +4,8 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "sfmm_fx_layout.hpp"
+
 namespace sfmm {
 
 std::vector<std::vector<double>> swap_matrices(int P)
@@ -159,6 +161,73 @@ HostTables build_tables(int P)
             }
     }
     return t;
+}
+
+namespace {
+
+void put_fx(int32_t *at, double v, int scale)
+{
+    const int64_t m = std::llround(std::ldexp(v, scale));
+    const int64_t h = (m + (int64_t(1) << 29)) >> 30;
+    at[0] = (int32_t)h;
+    at[1] = (int32_t)(m - h * (int64_t(1) << 30));
+}
+
+}  // namespace
+
+FxTables build_fx_tables(const HostTables &t, int G, int P)
+{
+    FxTables f;
+    f.P = P;
+    const int RS = G / 2;
+    f.woff.resize(P);
+    size_t tot = 0;
+    for (int n = 0; n < P; ++n) {
+        f.woff[n] = (int)tot;
+        tot += size_t((n + 2) / 2) * ((n + RS) / RS) * G;
+    }
+    f.W.assign(2 * tot, 0);
+    for (int n = 0; n < P; ++n) {
+        const int d = n + 1, NA = (d + RS - 1) / RS, cnt = (d + 1) / 2;
+        for (int tt = 0; tt < cnt; ++tt)
+            for (int q = 0; q < G; ++q)
+                for (int a = 0; a < NA; ++a) {
+                    const int part = q & 1, i = (q >> 1) + RS * a, j = ((i + n + part) & 1) + 2 * tt;
+                    const size_t in_slot = a / 2 * 2 + 1 < NA ? size_t(a / 2 * G + q) * 2 + (a & 1) : size_t(NA - 1) * G + q;
+                    put_fx(&f.W[2 * (f.woff[n] + size_t(tt) * NA * G + in_slot)], w_entry(t, n, part, i, j), 60);
+                }
+    }
+    f.hoff.resize(P);
+    tot = 0;
+    for (int m = 0; m < P; ++m) {
+        f.hoff[m] = (int)tot;
+        tot += size_t(P - m) * fx_hrow(P - m, G);
+    }
+    for (int op = 0; op < 3; ++op) {
+        f.H[op].assign(tot, 0.0);
+        for (int m = 0; m < P; ++m) {
+            const int HR = hrows(t.P - m, t.pad), hs = fx_hrow(P - m, G);
+            for (int k = 0; k < P - m; ++k)
+                for (int np = 0; np < P - m; ++np) {
+                    const int r = np % RS, b = np / RS;
+                    f.H[op][f.hoff[m] + size_t(k) * hs + b / 2 * G + 2 * r + (b & 1)] =
+                        t.H[op][t.hoff[m] + size_t(k) * HR + np];
+                }
+        }
+    }
+    return f;
+}
+
+std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count)
+{
+    std::vector<int32_t> out(4 * count);
+    for (size_t i = 0; i < count; ++i) {
+        int ex;
+        const double f = std::frexp(e[i], &ex);  // [1/2, 1)
+        put_fx(&out[4 * i], f, 60);
+        out[4 * i + 2] = ex;
+    }
+    return out;
 }
 
 }  // namespace sfmm

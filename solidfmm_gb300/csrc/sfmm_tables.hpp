@@ -18,6 +18,7 @@
 #pragma once
 
 #include <cstddef>
+#include <cstdint>
 #include <vector>
 
 namespace sfmm {
@@ -71,5 +72,28 @@ double w_entry(const HostTables &t, int n, int part, int i, int j);
 inline int hrows(int L, int pad) { return (L + pad - 1) & ~(pad - 1); }
 
 HostTables build_tables(int P);
+
+// Tables of the 60-bit fixed-point kernel for G threads per translation and
+// orders up to P, from the context's tables.
+struct FxTables {
+    int P = 0;
+    // Swap coefficients round(w 2^60) = h 2^30 + l, |l| <= 2^29, as (h, l)
+    // pairs; degree n at woff[n] (in pairs).  Lane q of the G lanes holds part
+    // q & 1 (W_R, W_I) of the rows i = (q >> 1) + (G/2) a, a < NA =
+    // ceil(d / (G/2)); slot t (column ((i + n + part) & 1) + 2t) lies at
+    // woff[n] + t NA G: for each pair of rows a = 2p, 2p + 1 the two
+    // coefficients of lane q at (p G + q) 2, for an odd last row lane q's at
+    // (NA - 1) G + q.  Slots t < (d + 1) / 2.
+    std::vector<int32_t> W;
+    std::vector<int> woff;
+    // z matrices in FP64: column m of op at hoff[m], row k of it
+    // (k - m) fx_hrow(P - m, G) further, output n' = m + r + (G/2) b at
+    // (b / 2) G + 2 r + (b & 1)
+    std::vector<double> H[3];
+    std::vector<int> hoff;
+};
+FxTables build_fx_tables(const HostTables &t, int G, int P);
+// positive edge factors as (h, l, exponent, 0): (h 2^30 + l) 2^(exponent - 60)
+std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count);
 
 }  // namespace sfmm

@@ -35,6 +35,7 @@
 
 #include "sfmm_arith.cuh"
 #include "sfmm_fixed.cuh"
+#include "sfmm_fx.cuh"
 #include "sfmm_params.hpp"
 
 namespace sfmm {
@@ -60,10 +61,13 @@ __device__ __forceinline__ void prefetch_l2(const void *ptr)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr));
 }
 
-template <int N>
-struct ic {
-    static constexpr int value = N;
-};
+// a table's lines loaded into L1, spread over the CTA's threads
+__device__ __forceinline__ void touch_tables(const void *t, int bytes)
+{
+    for (int o = threadIdx.x * 32; o < bytes; o += blockDim.x * 32) {
+        asm volatile("{\n\t.reg .b32 t;\n\tld.global.nc.b32 t, [%0];\n\t}" ::"l"(static_cast<const char *>(t) + o));
+    }
+}
 
 // Calls f(ic<na>) for na in 1..MAXN (warp-uniform switch).
 template <int MAXN, class F>
@@ -596,8 +600,8 @@ struct Geometry {
 // false for host memory read over the link, where both cost end-to-end rate.
 // WORK: tiles come from a work list (persistent launches of fused plans)
 // instead of a fixed stride over the batch.
-template <class A, int G, int ACC, bool FIX = false, bool HBM = true, bool WORK = false>
-__global__ void __launch_bounds__(256) k_translate(KParams p)
+template <class A, int G, int ACC, bool FIX, bool HBM, bool WORK>
+__device__ __forceinline__ void translate_body(const KParams &p)
 {
     using AR = arith<A>;
     using T = typename AR::T;
@@ -605,7 +609,9 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
     using Src = typename src_of<A>::type;
     static_assert(sizeof(S) == sizeof(Src), "buffer slots hold one source value");
     static_assert(32 % G == 0, "a translation's threads must share a warp");
-    static_assert(!FIX || AR::split, "fixed-point swaps are a float-float variant");
+    // block fixed point: 30-bit mantissas in the float-float kernel, 60-bit in FP64
+    constexpr bool FX = FIX && std::is_same<A, double>::value;
+    static_assert(!FIX || AR::split || FX, "fixed-point swaps are a float-float or FP64 variant");
 
     // Loads in flight per lane in the source gather and the target update,
     // measured on GB300 (M2L P=16, 10^6): 8 and 4 make the split kernel 2.2%
@@ -622,8 +628,9 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
     // inside the FP32 range at every geometry scale; shifts whose largest
     // component lies in [2, 4) run unscaled
     constexpr bool kScale = !std::is_same<A, double>::value;
-    constexpr int kGatherUnroll = kDeep ? 8 : 4;
+    constexpr int kGatherUnroll = kDeep || FX ? 8 : 4;
     constexpr int kAccUnroll = kDeep ? 4 : 1;
+    constexpr int kAccBatch = 5;
 
     extern __shared__ __align__(16) unsigned char smem[];
     const int TS = p.TS;
@@ -637,7 +644,8 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
     const unsigned FULL = 0xffffffffu;
 
     S *buf0 = reinterpret_cast<S *>(smem);
-    uint32_t *meta = reinterpret_cast<uint32_t *>(smem + (size_t)TS * p.spad * sizeof(S));
+    FxGeo *geo = reinterpret_cast<FxGeo *>(smem + (size_t)TS * p.spad * sizeof(S));  // FX only
+    uint32_t *meta = reinterpret_cast<uint32_t *>(smem + (size_t)TS * p.spad * sizeof(S) + (FX ? TS * sizeof(FxGeo) : 0));
     uint32_t *m_sidx = meta;
     uint32_t *m_tidx = meta + TS;
     uint32_t *m_pin = meta + 2 * TS;
@@ -651,6 +659,14 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
     const Src *src = reinterpret_cast<const Src *>(p.src);
     Src *dst = reinterpret_cast<Src *>(p.dst);
     const int op = p.op;
+    if constexpr (FX) {
+        // this order's tables into L1, all loads in flight at once (the
+        // transforms would meet them one miss after the other)
+        touch_tables(p.W, p.wbytes);
+        touch_tables(p.H, p.hbytes);
+        touch_tables(p.ein, P * (P + 1) / 2 * 16);
+        touch_tables(p.eout, P * (P + 1) / 2 * 16);
+    }
 
     for (long long tile = blockIdx.x;; tile += gridDim.x) {
         // this tile's range of the processing order: a fixed stride over the
@@ -679,11 +695,15 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
         uint32_t t = 0, si = 0, ti = 0;
         if (valid) t = p.perm ? p.perm[i] : (uint32_t)i;
         int pin = 0, pout = 0;
-        if (valid && t < p.nidx) {
+        double x = 0, y = 0, z = 1;
+        if (valid && t < p.nidx) {  // one round of independent loads
             si = p.sidx ? p.sidx[t] : t;
             ti = p.tidx ? p.tidx[t] : t;
             pin = (int)p.pin[t];
             pout = (int)p.pout[t];
+            x = p.shift[3 * (long long)t];
+            y = p.shift[3 * (long long)t + 1];
+            z = p.shift[3 * (long long)t + 2];
         }
         // malformed entries (the unchecked API's undefined behaviour) are
         // skipped and reported instead of touching memory out of bounds
@@ -691,12 +711,8 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
             if (q == 0) atomicOr(p.status, 1);
             valid = false;
             pin = pout = 0;
-        }
-        double x = 0, y = 0, z = 1;
-        if (valid) {
-            x = p.shift[3 * (long long)t];
-            y = p.shift[3 * (long long)t + 1];
-            z = p.shift[3 * (long long)t + 2];
+            x = y = 0;
+            z = 1;
         }
         if (op == OP_M2M) {  // M2M translates by the negated shift (translations.cpp:331-333)
             x = -x;
@@ -730,8 +746,15 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
             m_pin[slot] = (uint32_t)pin | ((uint32_t)(ks + 32768) << 16);  // order, and the scale above it
             m_pout[slot] = pout;
             m_id[slot] = ident_p;
+            if constexpr (FX) *reinterpret_cast<double3 *>(geo + slot) = make_double3(x, y, z);
         }
         __syncthreads();
+        if constexpr (FX) {  // one thread per translation: the others' lanes would only repeat it
+            if (tid < TS) {
+                const double3 v = *reinterpret_cast<const double3 *>(geo + tid);
+                fx_geometry(v.x, v.y, v.z, geo + tid);
+            }
+        }
 
         // 1. gather sources into the buffer (one warp per expansion, lanes over
         //    coefficients) in the arithmetic's storage format, zero past each
@@ -793,78 +816,121 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
         const int pin_w = __reduce_max_sync(FULL, pin);
         const int pout_w = __reduce_max_sync(FULL, pout);
 
-        // geometry (euler, microkernel_generic.cpp:37-97)
-        Geometry<AR, G, ACC, FIX> geo(x, y, z, q);
-        const Trig<AR, ACC> &tg = geo.tg;
-        const FixTrig<ACC> &tq = geo.tq;
-
-        // 2. forward transforms, degree by degree
-        const bool Lin = (op == OP_L2L);
-        // r-power scale of degree n: r^n (L input) or r^-(n+1) (M input).
-        // Float-float steps by repeated multiplication (FP32 pipe, error
-        // ~n 2^-48); FP64 and FP32 take every power from the FP64 product.
-        constexpr bool kFF = AR::split;
-        double rp = Lin ? 1.0 : geo.rinvd;
-        const double rpstep = Lin ? geo.rd : geo.rinvd;
-        T f = Lin ? AR::from_d(1.0) : geo.rinv;
-        const T rstep = Lin ? geo.r : geo.rinv;
-        for (int n = 0; n < pin_w; ++n) {
-            if (!kFF) f = AR::from_d(rp);
-            const T *ein = EIN + n * (n + 1) / 2;
-            if constexpr (FIX) {
-                const int *WRq = p.Wq + __ldg(p.woff + n);
-                dispatch<ACC>((n + G) / G, [&](auto na) {
-                    forward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, ein, f, q, tg, tq);
+        if constexpr (FX) {
+            const FxGeo &ge = geo[slot];
+            const int part = q & 1;
+            FxTrig<ACC> tg;
+            fx_powers<G / 2, ACC>(ge.ca, ge.sa, q >> 1, part, tg.ca, tg.sa);
+            fx_powers<G / 2, ACC>(ge.cb, ge.sb, q >> 1, part, tg.cb, tg.sb);
+            const fxs r{fx_split(ge.r), ge.re}, rinv{fx_split(ge.rinv), ge.rinve}, one{fx{1 << 29, 0}, 1};
+            const bool bad = ge.re == kFxBad;
+            const int2 *W = reinterpret_cast<const int2 *>(p.W);
+            const int4 *EIN = reinterpret_cast<const int4 *>(p.ein), *EOUT = reinterpret_cast<const int4 *>(p.eout);
+            const double *H = reinterpret_cast<const double *>(p.H);
+            // 2. forward transforms: r^n (L input) or r^-(n+1) (M input)
+            fxs f = op == OP_L2L ? one : rinv;
+            for (int n = 0; n < pin_w; ++n) {
+                dispatch<ACC>((n + G / 2) / (G / 2), [&](auto na) {
+                    forward_degree_fx<G, decltype(na)::value, ACC>(b, n, W + __ldg(p.woff + n), EIN + n * (n + 1) / 2, f,
+                                                                  bad, q, tg);
                 });
-            } else {
-                const T *WR = W + __ldg(p.woff + n);
-                dispatch<ACC>((n + G) / G, [&](auto na) {
-                    forward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, ein, f, q, tg);
+                f = fxs_mul(f, op == OP_L2L ? r : rinv);
+            }
+            // 3. z-translation (columns m >= min(P_in, P_out) of the outputs
+            // stay zero: their rows beyond P_in were zero-filled by the gather)
+            const int mend = min(pin_w, pout_w);
+            for (int m = 0; m < mend; ++m)
+                dispatch<ACC>((pout_w - m + G / 2 - 1) / (G / 2), [&](auto nb) {
+                    constexpr int NB = decltype(nb)::value;
+                    const double *Hm = H + __ldg(p.hoff + m);
+                    const int hs = fx_hrow(p.Ptab - m, G);
+                    if (op == OP_M2L) z_column_fx<G, NB>(b, Hm, hs, m, m, pin_w, pout_w, q);
+                    else if (op == OP_L2L) z_column_tri_fx<G, NB, true>(b, Hm, hs, m, pin_w, pout_w, q);
+                    else z_column_tri_fx<G, NB, false>(b, Hm, hs, m, mend, pout_w, q);
+                });
+            // 4. backward transforms: r^(n+1) (M output) or r^-n (L output)
+            f = op == OP_M2M ? r : one;
+            for (int n = 0; n < pout_w; ++n) {
+                dispatch<ACC>((n + G / 2) / (G / 2), [&](auto na) {
+                    backward_degree_fx<G, decltype(na)::value, ACC>(b, n, W + __ldg(p.woff + n), EOUT + n * (n + 1) / 2,
+                                                                   f, bad, q, tg);
+                });
+                f = fxs_mul(f, op == OP_M2M ? r : rinv);
+            }
+        } else {
+            // geometry (euler, microkernel_generic.cpp:37-97)
+            Geometry<AR, G, ACC, FIX> geo(x, y, z, q);
+            const Trig<AR, ACC> &tg = geo.tg;
+            const FixTrig<ACC> &tq = geo.tq;
+
+            // 2. forward transforms, degree by degree
+            const bool Lin = (op == OP_L2L);
+            // r-power scale of degree n: r^n (L input) or r^-(n+1) (M input).
+            // Float-float steps by repeated multiplication (FP32 pipe, error
+            // ~n 2^-48); FP64 and FP32 take every power from the FP64 product.
+            constexpr bool kFF = AR::split;
+            double rp = Lin ? 1.0 : geo.rinvd;
+            const double rpstep = Lin ? geo.rd : geo.rinvd;
+            T f = Lin ? AR::from_d(1.0) : geo.rinv;
+            const T rstep = Lin ? geo.r : geo.rinv;
+            for (int n = 0; n < pin_w; ++n) {
+                if (!kFF) f = AR::from_d(rp);
+                const T *ein = EIN + n * (n + 1) / 2;
+                if constexpr (FIX) {
+                    const int *WRq = p.Wq + __ldg(p.woff + n);
+                    dispatch<ACC>((n + G) / G, [&](auto na) {
+                        forward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, ein, f, q, tg, tq);
+                    });
+                } else {
+                    const T *WR = W + __ldg(p.woff + n);
+                    dispatch<ACC>((n + G) / G, [&](auto na) {
+                        forward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, ein, f, q, tg);
+                    });
+                }
+                if (kFF) f = AR::mul(f, rstep);
+                if (!kFF) rp *= rpstep;
+            }
+
+            // 3. z-translation, column by column.  Columns m >= min(P_in, P_out)
+            //    of the outputs stay zero (trans2swap_buf, microkernel_generic.cpp:308-338):
+            //    their rows beyond P_in were zero-filled by the gather.
+            const int nout_w = pout_w;
+            const int mend = min(pin_w, pout_w);
+            for (int m = 0; m < mend; ++m) {
+                const int HR = (p.Ptab - m + p.rowpad - 1) & ~(p.rowpad - 1);
+                const T *Hm = H + __ldg(p.hoff + m);
+                // M2M only needs inputs k <= n' and L2L only k >= n'
+                const int kbeg = (op == OP_L2L) ? m + q : m;
+                const int kend = (op == OP_M2M) ? min(pin_w, nout_w) : pin_w;
+                dispatch<ACC>((nout_w - m + G - 1) / G, [&](auto na) {
+                    z_column<AR, G, decltype(na)::value>(b, Hm, HR, m, kbeg, kend, nout_w, q);
                 });
             }
-            if (kFF) f = AR::mul(f, rstep);
-            if (!kFF) rp *= rpstep;
-        }
 
-        // 3. z-translation, column by column.  Columns m >= min(P_in, P_out)
-        //    of the outputs stay zero (trans2swap_buf, microkernel_generic.cpp:308-338):
-        //    their rows beyond P_in were zero-filled by the gather.
-        const int nout_w = pout_w;
-        const int mend = min(pin_w, pout_w);
-        for (int m = 0; m < mend; ++m) {
-            const int HR = (p.Ptab - m + p.rowpad - 1) & ~(p.rowpad - 1);
-            const T *Hm = H + __ldg(p.hoff + m);
-            // M2M only needs inputs k <= n' and L2L only k >= n'
-            const int kbeg = (op == OP_L2L) ? m + q : m;
-            const int kend = (op == OP_M2M) ? min(pin_w, nout_w) : pin_w;
-            dispatch<ACC>((nout_w - m + G - 1) / G, [&](auto na) {
-                z_column<AR, G, decltype(na)::value>(b, Hm, HR, m, kbeg, kend, nout_w, q);
-            });
-        }
-
-        // 4. backward transforms
-        const bool Mout = (op == OP_M2M);
-        double rq = Mout ? geo.rd : 1.0;  // r^(n+1) (M output) or r^-n (L output)
-        const double rqstep = Mout ? geo.rd : geo.rinvd;
-        T fo = Mout ? geo.r : AR::from_d(1.0);
-        const T qstep = Mout ? geo.r : geo.rinv;
-        for (int n = 0; n < nout_w; ++n) {
-            if (!kFF) fo = AR::from_d(rq);
-            const T f = fo;
-            const T *eo = EOUT + n * (n + 1) / 2;
-            if constexpr (FIX) {
-                const int *WRq = p.Wq + __ldg(p.woff + n);
-                dispatch<ACC>((n + G) / G, [&](auto na) {
-                    backward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, eo, f, q, tg, tq);
-                });
-            } else {
-                const T *WR = W + __ldg(p.woff + n);
-                dispatch<ACC>((n + G) / G, [&](auto na) {
-                    backward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, eo, f, q, tg);
-                });
+            // 4. backward transforms
+            const bool Mout = (op == OP_M2M);
+            double rq = Mout ? geo.rd : 1.0;  // r^(n+1) (M output) or r^-n (L output)
+            const double rqstep = Mout ? geo.rd : geo.rinvd;
+            T fo = Mout ? geo.r : AR::from_d(1.0);
+            const T qstep = Mout ? geo.r : geo.rinv;
+            for (int n = 0; n < nout_w; ++n) {
+                if (!kFF) fo = AR::from_d(rq);
+                const T f = fo;
+                const T *eo = EOUT + n * (n + 1) / 2;
+                if constexpr (FIX) {
+                    const int *WRq = p.Wq + __ldg(p.woff + n);
+                    dispatch<ACC>((n + G) / G, [&](auto na) {
+                        backward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, eo, f, q, tg, tq);
+                    });
+                } else {
+                    const T *WR = W + __ldg(p.woff + n);
+                    dispatch<ACC>((n + G) / G, [&](auto na) {
+                        backward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, eo, f, q, tg);
+                    });
+                }
+                if (kFF) fo = AR::mul(fo, qstep);
+                if (!kFF) rq *= rqstep;
             }
-            if (kFF) fo = AR::mul(fo, qstep);
-            if (!kFF) rq *= rqstep;
         }
         __syncthreads();
 
@@ -882,6 +948,20 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
             // degree j times lambda^j (multipoles) or lambda^-(j+1) (locals)
             const int ksa = (int)(m_pin[s] >> 16) - 32768;
             const int eo = op == OP_M2M ? ksa : -ksa, eo0 = op == OP_M2M ? 0 : -ksa;
+            if constexpr (FX) {
+                // kAccBatch target loads in flight per lane
+                if (!p.atomic && !pid) {
+                    for (int c0 = lane; c0 < cnt; c0 += 32 * kAccBatch) {
+                        double v[kAccBatch];
+#pragma unroll
+                        for (int u = 0; u < kAccBatch; ++u) v[u] = c0 + 32 * u < cnt ? __ldcs(dp + c0 + 32 * u) : 0.0;
+#pragma unroll
+                        for (int u = 0; u < kAccBatch; ++u)
+                            if (c0 + 32 * u < cnt) __stcs(dp + c0 + 32 * u, v[u] + bp[c0 + 32 * u]);
+                    }
+                    continue;
+                }
+            }
 #pragma unroll(kAccUnroll)
             for (int c = lane; c < cnt; c += 32) {
                 const int j = kScale ? degree_at(c) : 0;
@@ -914,6 +994,20 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
         }
         __syncthreads();
     }
+}
+
+template <class A, int G, int ACC, bool FIX = false, bool HBM = true, bool WORK = false>
+__global__ void __launch_bounds__(256) k_translate(KParams p)
+{
+    translate_body<A, G, ACC, FIX, HBM, WORK>(p);
+}
+
+constexpr int fx_blocks(int acc) { return acc <= 4 ? 5 : acc <= 6 ? 4 : 2; }
+// FP64 in 60-bit block fixed point
+template <int G, int ACC, bool HBM = true, bool WORK = false>
+__global__ void __launch_bounds__(kFxThreads, fx_blocks(ACC)) k_translate_fx(KParams p)
+{
+    translate_body<double, G, ACC, true, HBM, WORK>(p);
 }
 
 }  // namespace sfmm
