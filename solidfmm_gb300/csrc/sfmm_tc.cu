@@ -180,9 +180,11 @@ cudaError_t tc_prepare(TcDevTables **out, int mode, const HostTables &host)
     }
     if (e == cudaSuccess) {
         const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        if (mode == 0) e = cudaFuncSetAttribute(k_translate_tc<0, kTcGroups>, at, smem_bytes<0>(Pt));
-        else if (mode == 1) e = cudaFuncSetAttribute(k_translate_tc<1, kTcGroups>, at, smem_bytes<1>(Pt));
-        else e = cudaFuncSetAttribute(k_translate_tc<2, kTcGroups>, at, smem_bytes<2>(Pt));
+        // the limit belongs to the kernel, not to this context: a context of
+        // a lower order must not shrink it for the others
+        if (mode == 0) e = cudaFuncSetAttribute(k_translate_tc<0, kTcGroups>, at, smem_bytes<0>(kTcMaxOrder));
+        else if (mode == 1) e = cudaFuncSetAttribute(k_translate_tc<1, kTcGroups>, at, smem_bytes<1>(kTcMaxOrder));
+        else e = cudaFuncSetAttribute(k_translate_tc<2, kTcGroups>, at, smem_bytes<2>(kTcMaxOrder));
     }
     if (e != cudaSuccess) {
         tc_release(t);
