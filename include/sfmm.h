@@ -46,8 +46,9 @@ typedef enum { SFMM_F32 = 0, SFMM_F64 = 1 } sfmm_dtype;
 typedef enum { SFMM_M2M = 0, SFMM_M2L = 1, SFMM_L2L = 2 } sfmm_op;
 
 /* Arithmetic of the translation kernels.
- * PLAIN:    the storage type's own arithmetic (FP64 for SFMM_F64, FP32 for
- *           SFMM_F32).
+ * PLAIN:    the storage type's own accuracy (SFMM_F64: rotations and swaps in
+ *           60-bit block fixed point up to order 32, FP64 otherwise; SFMM_F32:
+ *           FP32).
  * SPLIT:    FP64 expansions in, FP64 accumulation out, the translation itself
  *           on the FP32 and integer pipes with relative error <= 1e-7 in the
  *           orthonormal (Schmidt) basis: swaps and polar rotations in block
@@ -57,8 +58,8 @@ typedef enum { SFMM_M2M = 0, SFMM_M2L = 1, SFMM_L2L = 2 } sfmm_op;
  *           M2M batches with an order bound above 18 run the SPLIT_FF
  *           arithmetic: there the rotation method's error growth with the
  *           degree would take 30-bit mantissas past 1e-7.
- * SPLIT_FF: the same with float-float (double-FP32, ~2^-44 per operation)
- *           for every stage: relative error ~1e-13 at order 16.
+ * SPLIT_FF: FP64's own accuracy for the whole translation (orders <= 28);
+ *           runs the PLAIN kernel of an SFMM_F64 context.
  * TC_TF32:  the tensor-core kernel (tcgen05, one thread per translation,
  *           128 translations per MMA tile): every swap and z-translation is
  *           an MMA against constant matrices held in shared memory, with both

@@ -235,14 +235,20 @@ int arith_of(sfmm_context *c, int precision, Arith *out)
 // fixed-point rotations for M2L and L2L up to order 28 and M2M up to order
 // 18.  Past that the rotation method's own error growth with the degree
 // (about 1.35x per degree for M2M, in every arithmetic) pushes 30-bit
-// mantissas above 1e-7, and the batch runs in float-float instead.
+// mantissas above 1e-7, and the batch runs as SFMM_SPLIT_FF instead.
 constexpr int kFixedM2MOrder = 18;
+// SFMM_SPLIT_FF runs the FP64 kernel, whose 60-bit fixed point needs no more
+// time than float-float did and rounds less: M2L at P=16 86.9 M/s and 3e-15
+// against 80.7 M/s and 7e-14, P=6 605 / 519, P=24 25.2 / 24.0, P=28 14.0 / 14.2.
+// Orders above kMaxFloatOrder, which the mode never took, keep Arith::FF and
+// are refused by prepare_launch.
 // The tensor-core kernel holds a tile's expansions in tensor memory up to
 // order 16; batches with a larger order bound run the split kernel.
 Arith resolve_arith(Arith a, int op, int Pbound)
 {
     if (is_tc(a) && Pbound > tc_max_order()) a = Arith::FFQ;
-    if (a == Arith::FFQ && op == SFMM_M2M && Pbound > kFixedM2MOrder) return Arith::FF;
+    if (a == Arith::FFQ && op == SFMM_M2M && Pbound > kFixedM2MOrder) a = Arith::FF;
+    if (a == Arith::FF && Pbound <= kMaxFloatOrder) a = Arith::F64;
     return a;
 }
 
@@ -270,14 +276,14 @@ int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *sh
         }
         return SFMM_OK;
     }
+    if (a != Arith::F64 && Pbound > kMaxFloatOrder)
+        return fail(c, SFMM_UNSUPPORTED, "order %d exceeds %d, the limit of FP32-range arithmetic", Pbound, kMaxFloatOrder);
     const auto key = std::make_tuple(op, (int)a, Pbound);
     auto it = c->shapes.find(key);
     if (it == c->shapes.end()) it = c->shapes.emplace(key, best_shape(a, Pbound, default_group(a, Pbound))).first;
     if (shape) *shape = it->second;
     if (it->second.acc == 0)
         return fail(c, SFMM_UNSUPPORTED, "order %d exceeds the GPU kernels' limit %d", Pbound, kMaxKernelOrder);
-    if (a != Arith::F64 && Pbound > kMaxFloatOrder)
-        return fail(c, SFMM_UNSUPPORTED, "order %d exceeds %d, the limit of FP32-range arithmetic", Pbound, kMaxFloatOrder);
     return ensure_shape_tables(c, a, it->second);
 }
 
@@ -451,7 +457,7 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
 // 8 from a sweep on GB300 (M2L, uniform orders 2..32, both group sizes): 8
 // threads pay off once the per-translation buffers limit the SM to a few
 // warps and the group's own arithmetic is cheap enough to leave latency
-// exposed (FP32 from 17, both split modes from 14).  FP64 (60-bit fixed point)
+// exposed (FP32 from 17, split from 14).  FP64 (60-bit fixed point)
 // from 13, where four threads need more rows than fit the registers of a full
 // SM: M2L at P=12 189 M/s with 4 and 150 with 8, at P=13 89 and 125.
 int default_group(Arith a, int P)
@@ -460,7 +466,6 @@ int default_group(Arith a, int P)
     switch (a) {
     case Arith::F64: return P >= 13 ? 8 : 4;
     case Arith::F32: return P >= 17 ? 8 : 4;
-    case Arith::FF: return P >= 14 ? 8 : 4;
     case Arith::FFQ: return P >= 14 ? 8 : 4;
     }
     return 4;
@@ -501,11 +506,9 @@ cudaError_t launch_translate_64(const KParams &, const LaunchShape &, int, cudaS
 cudaError_t launch_translate_fx(const KParams &, const LaunchShape &, int, cudaStream_t);
 int occupancy_fx64(const LaunchShape &);
 cudaError_t launch_translate_32(const KParams &, const LaunchShape &, int, cudaStream_t);
-cudaError_t launch_translate_ff(const KParams &, const LaunchShape &, int, cudaStream_t);
 cudaError_t launch_translate_ffq(const KParams &, const LaunchShape &, int, cudaStream_t);
 int occupancy_64(const LaunchShape &);
 int occupancy_32(const LaunchShape &);
-int occupancy_ff(const LaunchShape &);
 int occupancy_ffq(const LaunchShape &);
 
 cudaError_t launch_translate(Arith a, const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
@@ -514,7 +517,7 @@ cudaError_t launch_translate(Arith a, const KParams &p, const LaunchShape &s, in
     case Arith::F64: return s.fx ? launch_translate_fx(p, s, grid, st) : launch_translate_64(p, s, grid, st);
     case Arith::F32: return launch_translate_32(p, s, grid, st);
     case Arith::FFQ: return launch_translate_ffq(p, s, grid, st);
-    default: return launch_translate_ff(p, s, grid, st);
+    default: return cudaErrorInvalidValue;
     }
 }
 
@@ -524,7 +527,7 @@ int translate_blocks_per_sm(Arith a, const LaunchShape &s)
     case Arith::F64: return s.fx ? occupancy_fx64(s) : occupancy_64(s);
     case Arith::F32: return occupancy_32(s);
     case Arith::FFQ: return occupancy_ffq(s);
-    default: return occupancy_ff(s);
+    default: return 1;  // Arith::FF above its orders: a shape to pin, no kernel
     }
 }
 

@@ -433,37 +433,63 @@ __device__ __forceinline__ void backward_degree_fx(double *b, int n, const int2 
     __syncwarp();
 }
 
-// One z-translation column m in FP64: outputs n' = m + r + RS b (b < NB) of
-// the lane's part, in(k, m) read once per row for all of them.  H_m lies row
-// by row (k), in each row pairs of blocks lane by lane (double2), hs doubles
-// per row.
-template <int G, int NB>
-__device__ __forceinline__ void z_column_fx(double *b, const double *__restrict__ Hm, int hs, int m, int kbeg, int kend,
-                                            int nout, int q)
+// V = 16 / sizeof(T) consecutive row blocks of a z matrix row come by one load
+template <class T>
+constexpr int kZVec = 16 / (int)sizeof(T);
+template <class T>
+struct zvec;
+template <>
+struct zvec<double> {
+    using type = double2;
+    static __device__ __forceinline__ void get(const type &v, double *w)
+    {
+        w[0] = v.x;
+        w[1] = v.y;
+    }
+};
+template <>
+struct zvec<float> {
+    using type = float4;
+    static __device__ __forceinline__ void get(const type &v, float *w)
+    {
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+    }
+};
+// blocks [B0, B1) of one row into w[B0 ..] (w has room for whole vectors)
+template <class T, int RS, int B0, int B1, int N>
+__device__ __forceinline__ void z_load(const T *h, T (&w)[N])
 {
-    constexpr int RS = G / 2;
+    constexpr int V = kZVec<T>;
+#pragma unroll
+    for (int i = B0 / V; i < (B1 + V - 1) / V; ++i) {
+        if (B1 - i * V == 1) w[i * V] = __ldg(h + i * RS * V);
+        else zvec<T>::get(__ldg(reinterpret_cast<const typename zvec<T>::type *>(h + i * RS * V)), w + i * V);
+    }
+}
+
+// One z-translation column m: outputs n' = m + r + RS b (b < NB) of the
+// lane's part, in(k, m) read once per row for all of them.  H_m lies row by
+// row (k), in each row vectors of V blocks lane by lane, hs elements per row.
+template <class T, int G, int NB>
+__device__ __forceinline__ void z_column_part(T *b, const T *__restrict__ Hm, int hs, int m, int kend, int nout, int q)
+{
+    constexpr int RS = G / 2, V = kZVec<T>, NW = (NB + V - 1) / V * V;
     const int r = q >> 1, part = q & 1;
-    double acc[NB];
+    T acc[NB];
 #pragma unroll
-    for (int i = 0; i < NB; ++i) acc[i] = 0.0;
-    const double *h = Hm + (long long)(kbeg - m) * hs + 2 * r;
-    int o = kbeg * (kbeg + 1) + m + part * (kbeg + 1);
-    int step = 2 * (kbeg + 1) + part;
-    auto load = [&](double (&w)[NB]) {
-#pragma unroll
-        for (int i = 0; i < NB / 2; ++i) {
-            const double2 u = __ldg(reinterpret_cast<const double2 *>(h + i * G));
-            w[2 * i] = u.x;
-            w[2 * i + 1] = u.y;
-        }
-        if constexpr (NB & 1) w[NB - 1] = __ldg(h + (NB / 2) * G);
-    };
-    double wn[NB], xn = b[o];
-    load(wn);
+    for (int i = 0; i < NB; ++i) acc[i] = 0;
+    const T *h = Hm + V * r;
+    int o = m * (m + 1) + m + part * (m + 1);
+    int step = 2 * (m + 1) + part;
+    T wn[NW], xn = b[o];
+    z_load<T, RS, 0, NB>(h, wn);
 #pragma unroll 2
-    for (int k = kbeg; k < kend; ++k) {  // row k+1's operands load before row k's multiply-adds
-        const double x = xn;
-        double w[NB];
+    for (int k = m; k < kend; ++k) {  // row k+1's operands load before row k's multiply-adds
+        const T x = xn;
+        T w[NB];
 #pragma unroll
         for (int i = 0; i < NB; ++i) w[i] = wn[i];
         if (k + 1 < kend) {
@@ -472,7 +498,7 @@ __device__ __forceinline__ void z_column_fx(double *b, const double *__restrict_
             h += hs;
         }
         xn = b[o];
-        load(wn);
+        z_load<T, RS, 0, NB>(h, wn);
 #pragma unroll
         for (int i = 0; i < NB; ++i) acc[i] = fma(w[i], x, acc[i]);
     }
@@ -490,41 +516,38 @@ __device__ __forceinline__ void z_column_fx(double *b, const double *__restrict_
 // rows, k = m + r + j upwards (L2L) or k = m + r + RS (NB - 1) - j downwards
 // (M2M), so that with every RS rows one more block of outputs joins, for all
 // lanes at once: 40 of 64 multiply-adds of a column of 16 remain.
-template <int G, int NB, bool UP>
-__device__ __forceinline__ void z_column_tri_fx(double *b, const double *__restrict__ Hm, int hs, int m, int kend,
-                                                int nout, int q)
+template <class T, int G, int NB, bool UP>
+__device__ __forceinline__ void z_column_tri(T *b, const T *__restrict__ Hm, int hs, int m, int kend, int nout, int q)
 {
-    constexpr int RS = G / 2, D = UP ? 1 : -1;
+    constexpr int RS = G / 2, D = UP ? 1 : -1, V = kZVec<T>, NW = (NB + V - 1) / V * V;
     const int r = q >> 1, part = q & 1;
-    double acc[NB];  // block i of the order in which they join
+    T acc[NB];
 #pragma unroll
-    for (int i = 0; i < NB; ++i) acc[i] = 0.0;
+    for (int i = 0; i < NB; ++i) acc[i] = 0;
     // rows that no lane has: above kend on the way down
     int j = UP ? 0 : max(0, m + RS * (NB - 1) - kend + 1);
     const int rows = UP ? kend - m : RS * NB;
     int k = m + r + (UP ? 0 : RS * (NB - 1) - j);
-    const double *h = Hm + (long long)(k - m) * hs + 2 * r;
+    const T *h = Hm + (long long)(k - m) * hs + V * r;
     int o = k * (k + 1) + m + part * (k + 1);
     int step = UP ? 2 * (k + 1) + part : 2 * k + part;  // to the next row (UP) or the previous one
-    auto row = [&](auto nb) {
-        constexpr int N = decltype(nb)::value;
-        const bool on = UP ? k < kend : k < kend && k >= m;
-        const double x = on ? b[o] : 0.0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const int blk = UP ? i : NB - 1 - i;
-            acc[i] = fma(on ? __ldg(h + blk / 2 * G + (blk & 1)) : 0.0, x, acc[i]);
-        }
-        k += D;
-        o += D * step;
-        step += 2 * D;
-        h += D * hs;
-    };
     auto stage = [&](auto nb) {
-        constexpr int N = decltype(nb)::value;
+        constexpr int N = decltype(nb)::value, B0 = UP ? 0 : NB - N, B1 = UP ? N : NB;  // blocks at work
         const int end = N < NB ? min(RS * N, rows) : rows;
 #pragma unroll 2
-        for (; j < end; ++j) row(nb);
+        for (; j < end; ++j) {
+            if (UP ? k < kend : k < kend && k >= m) {
+                const T x = b[o];
+                T w[NW];
+                z_load<T, RS, B0, B1>(h, w);
+#pragma unroll
+                for (int i = B0; i < B1; ++i) acc[i] = fma(w[i], x, acc[i]);
+            }
+            k += D;
+            o += D * step;
+            step += 2 * D;
+            h += D * hs;
+        }
     };
     stage(ic<1>{});
     if constexpr (NB >= 2) stage(ic<2>{});
@@ -537,10 +560,19 @@ __device__ __forceinline__ void z_column_tri_fx(double *b, const double *__restr
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-        const int np = m + r + RS * (UP ? i : NB - 1 - i);
+        const int np = m + r + RS * i;
         if (np < nout) b[np * (np + 1) + m + part * (np + 1)] = acc[i];
     }
     __syncwarp();
+}
+
+// Column m of operator op.
+template <class T, int G, int NB>
+__device__ __forceinline__ void z_column_op(int op, T *b, const T *__restrict__ Hm, int hs, int m, int pin, int pout, int q)
+{
+    if (op == OP_M2L) z_column_part<T, G, NB>(b, Hm, hs, m, pin, pout, q);
+    else if (op == OP_L2L) z_column_tri<T, G, NB, true>(b, Hm, hs, m, pin, pout, q);
+    else z_column_tri<T, G, NB, false>(b, Hm, hs, m, min(pin, pout), pout, q);
 }
 
 }  // namespace sfmm

@@ -10,8 +10,8 @@
 
 namespace sfmm {
 
-// doubles per row (input degree) of a z matrix with L outputs, for G threads
-// per translation: pairs of G/2-row blocks
-SFMM_HD constexpr int fx_hrow(int L, int G) { return ((L + G / 2 - 1) / (G / 2) + 1) / 2 * G; }
+// elements per row (input degree) of a z matrix with L outputs, for G threads
+// per translation: vectors of V blocks of G/2 rows
+SFMM_HD constexpr int fx_hrow(int L, int G, int V = 2) { return ((L + G / 2 - 1) / (G / 2) + V - 1) / V * (G / 2) * V; }
 
 }  // namespace sfmm

@@ -1,5 +1,5 @@
 // Explicit instantiation of the fused translation kernel for one arithmetic
-// type; included by sfmm_k64.cu, sfmm_k32.cu, sfmm_kff.cu and sfmm_kffq.cu
+// type; included by sfmm_k64.cu, sfmm_k32.cu, sfmm_kffq.cu and sfmm_kfx.cu
 // (one translation unit each, compiled in parallel).  Instances: group size G
 // in {4, 8, 32} and accumulator blocks ACC = ceil(P / G) rounded up to an
 // instantiated size; the fixed-point float-float variant (orders <= 28) has

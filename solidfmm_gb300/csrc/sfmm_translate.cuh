@@ -841,12 +841,8 @@ __device__ __forceinline__ void translate_body(const KParams &p)
             const int mend = min(pin_w, pout_w);
             for (int m = 0; m < mend; ++m)
                 dispatch<ACC>((pout_w - m + G / 2 - 1) / (G / 2), [&](auto nb) {
-                    constexpr int NB = decltype(nb)::value;
-                    const double *Hm = H + __ldg(p.hoff + m);
-                    const int hs = fx_hrow(p.Ptab - m, G);
-                    if (op == OP_M2L) z_column_fx<G, NB>(b, Hm, hs, m, m, pin_w, pout_w, q);
-                    else if (op == OP_L2L) z_column_tri_fx<G, NB, true>(b, Hm, hs, m, pin_w, pout_w, q);
-                    else z_column_tri_fx<G, NB, false>(b, Hm, hs, m, mend, pout_w, q);
+                    z_column_op<double, G, decltype(nb)::value>(op, b, H + __ldg(p.hoff + m), fx_hrow(p.Ptab - m, G), m,
+                                                                pin_w, pout_w, q);
                 });
             // 4. backward transforms: r^(n+1) (M output) or r^-n (L output)
             f = op == OP_M2M ? r : one;
