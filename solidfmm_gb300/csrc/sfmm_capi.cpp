@@ -165,38 +165,60 @@ int ensure_tables(sfmm_context *c, Arith a)
 }
 
 
-// Tables of the 60-bit fixed-point kernel for G threads per translation
-// (orders up to 32), once per context.
-int ensure_fx(sfmm_context *c, int G)
+namespace {
+
+cudaError_t put(void **dst, const void *src, size_t bytes)
 {
-    FxDevTables &t = c->fxt[G == 8];
+    cudaError_t e = cudaMalloc(dst, bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+    return e;
+}
+
+// the tables of one group size: swap coefficients of wsize bytes per woff unit
+template <class T>
+cudaError_t put_fx(FxDevTables &t, const T &h, int P, size_t wsize)
+{
+    cudaError_t e = put(&t.W, h.W.data(), h.W.size() * sizeof(h.W[0]));
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k].data(), h.H[k].size() * sizeof(h.H[k][0]));
+    if (e == cudaSuccess) e = put((void **)&t.woff, h.woff.data(), h.woff.size() * sizeof(int));
+    if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff.data(), h.hoff.size() * sizeof(int));
+    t.wend.assign(P + 1, (int)(h.W.size() * sizeof(h.W[0])));
+    for (int n = 0; n < P; ++n) t.wend[n] = (int)(h.woff[n] * wsize);
+    t.hbytes = (int)(h.H[0].size() * sizeof(h.H[0][0]));
+    t.P = P;
+    return e;
+}
+
+}  // namespace
+
+// Tables of the 60-bit fixed-point kernel (FP64) or of the FP32 kernel for G
+// threads per translation (orders up to 32), once per context.
+int ensure_fx(sfmm_context *c, Arith a, int G)
+{
+    FxDevTables &t = (a == Arith::F32 ? c->f32t : c->fxt)[G == 8];
     if (t.ready) return SFMM_OK;
     const int P = std::min(c->P, 32);
-    auto put = [](void **dst, const void *src, size_t bytes) {
-        cudaError_t e = cudaMalloc(dst, bytes);
-        if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
-        return e;
-    };
     cudaError_t e = cudaSuccess;
     try {
         const std::vector<double> *ev[4] = {&c->host.e_in_M, &c->host.e_in_L, &c->host.e_out_L, &c->host.e_out_M};
+        const size_t ne = (size_t)P * (P + 1) / 2;
         for (int k = 0; k < 4 && e == cudaSuccess; ++k) {
-            if (c->fx_edge[k]) continue;
-            const auto v = fx_edges(*ev[k], (size_t)P * (P + 1) / 2);
-            e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(int32_t));
+            if (c->fx_edge[k]) continue;  // a context has one data type
+            if (a == Arith::F32) {
+                const std::vector<float> v(ev[k]->begin(), ev[k]->begin() + ne);
+                e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(float));
+            } else {
+                const auto v = fx_edges(*ev[k], ne);
+                e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(int32_t));
+            }
             if (e != cudaSuccess && c->fx_edge[k]) {
                 cudaFree(c->fx_edge[k]);
                 c->fx_edge[k] = nullptr;
             }
         }
-        const FxTables h = build_fx_tables(c->host, G, P);
-        t.wend.assign(P + 1, (int)(h.W.size() * sizeof(int32_t)));
-        for (int n = 0; n < P; ++n) t.wend[n] = h.woff[n] * 8;
-        t.hbytes = (int)(h.H[0].size() * sizeof(double));
-        if (e == cudaSuccess) e = put(&t.W, h.W.data(), h.W.size() * sizeof(int32_t));
-        for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k].data(), h.H[k].size() * sizeof(double));
-        if (e == cudaSuccess) e = put((void **)&t.woff, h.woff.data(), h.woff.size() * sizeof(int));
-        if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff.data(), h.hoff.size() * sizeof(int));
+        if (e == cudaSuccess)
+            e = a == Arith::F32 ? put_fx(t, build_f32_tables(c->host, G, P), P, sizeof(float))
+                                : put_fx(t, build_fx_tables(c->host, G, P), P, 2 * sizeof(int32_t));
     } catch (const std::bad_alloc &) {
         free_fx(t);
         return fail(c, SFMM_OOM, "operator tables");
@@ -205,7 +227,6 @@ int ensure_fx(sfmm_context *c, int G)
         free_fx(t);  // a partial set is retried from scratch on the next call
         return cuda_fail(c, e, "table upload");
     }
-    t.P = P;
     t.ready = true;
     return SFMM_OK;
 }
@@ -255,7 +276,7 @@ Arith resolve_arith(Arith a, int op, int Pbound)
 // the device tables that a launch of this shape reads (setup_mtx held)
 static int ensure_shape_tables(sfmm_context *c, Arith a, const LaunchShape &s)
 {
-    return s.fx ? ensure_fx(c, s.G) : ensure_tables(c, a);
+    return s.fx ? ensure_fx(c, a, s.G) : ensure_tables(c, a);
 }
 
 int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *shape)
@@ -362,7 +383,7 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
         return SFMM_OK;
     }
     if (s.fx) {
-        const FxDevTables &t = c->fxt[s.G == 8];
+        const FxDevTables &t = (a == Arith::F32 ? c->f32t : c->fxt)[s.G == 8];
         p.W = t.W;
         p.woff = t.woff;
         p.hoff = t.hoff;
@@ -420,19 +441,20 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     int acc = (P + G - 1) / G;
     if (G == 4) acc = acc <= 2 ? 2 : (acc <= 4 ? 4 : (acc <= 6 ? 6 : 8));
     if (G == 32) acc = acc <= 2 ? 2 : 3;
-    // FP64 up to order 32 runs in 60-bit fixed point, rows in steps of G/2;
-    // four threads per translation only up to order 16 (more rows than their
-    // registers hold: above, a request for 4 runs 8)
-    s.fx = a == Arith::F64 && G != 32;
+    // FP64 (in 60-bit fixed point) and FP32 up to order 32: rows in steps of
+    // G/2; four threads per translation only up to order 16 (more rows than
+    // their registers hold: above, a request for 4 runs 8)
+    s.fx = (a == Arith::F64 || a == Arith::F32) && G != 32;
     if (s.fx) {
-        if (P > 16 && G == 4) {
+        if (P > 16 && G == 4 && a == Arith::F64) {
             G = 8;
             ts /= 2;
             if (ts < 32 / G || ts % (32 / G)) return s;
         }
         if (G * ts > kFxThreads) return LaunchShape{};
         acc = (P + G / 2 - 1) / (G / 2);
-        acc = G == 4 ? (acc <= 4 ? 4 : acc <= 6 ? 6 : 8) : (acc + 1) / 2 * 2;
+        if (a == Arith::F32) acc = acc <= 4 ? 4 : acc <= 6 ? 6 : acc <= 8 ? 8 : acc <= 10 ? 10 : 14;
+        else acc = G == 4 ? (acc <= 4 ? 4 : acc <= 6 ? 6 : 8) : (acc + 1) / 2 * 2;
     }
     s.G = G;
     s.acc = acc;
@@ -457,7 +479,8 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
 // 8 from a sweep on GB300 (M2L, uniform orders 2..32, both group sizes): 8
 // threads pay off once the per-translation buffers limit the SM to a few
 // warps and the group's own arithmetic is cheap enough to leave latency
-// exposed (FP32 from 17, split from 14).  FP64 (60-bit fixed point)
+// exposed (split from 14; FP32 from 15: M2L at P=14 338 M/s with 4 and 311 with 8,
+// at P=16 251 and 266, at P=20 136 and 145).  FP64 (60-bit fixed point)
 // from 13, where four threads need more rows than fit the registers of a full
 // SM: M2L at P=12 189 M/s with 4 and 150 with 8, at P=13 89 and 125.
 int default_group(Arith a, int P)
@@ -465,7 +488,7 @@ int default_group(Arith a, int P)
     if (P > 32) return 32;
     switch (a) {
     case Arith::F64: return P >= 13 ? 8 : 4;
-    case Arith::F32: return P >= 17 ? 8 : 4;
+    case Arith::F32: return P >= 15 ? 8 : 4;
     case Arith::FFQ: return P >= 14 ? 8 : 4;
     }
     return 4;
@@ -595,6 +618,7 @@ void sfmm_destroy(sfmm_context *c)
     for (auto &t : c->tab) free_tables(t);
     for (auto &t : c->tc) tc_release(t);
     for (auto &t : c->fxt) free_fx(t);
+    for (auto &t : c->f32t) free_fx(t);
     for (void *p : c->fx_edge)
         if (p) cudaFree(p);
     for (int k = 0; k < 3; ++k) {
@@ -679,7 +703,7 @@ int sfmm_set_group(sfmm_context *c, int precision, size_t order_bound, int group
     }
     std::lock_guard<std::mutex> lk2(c->setup_mtx);
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
-        if (s[op - SFMM_M2M].fx && (st = ensure_fx(c, group))) return st;  // before a capture may launch it
+        if (s[op - SFMM_M2M].fx && (st = ensure_fx(c, resolve_arith(a, op, Pb), s[op - SFMM_M2M].G))) return st;  // before a capture may launch it
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
         c->shapes[std::make_tuple(op, (int)resolve_arith(a, op, Pb), Pb)] = s[op - SFMM_M2M];
     return SFMM_OK;

@@ -31,9 +31,9 @@ struct DevTables {
     bool ready = false;
 };
 
-// device tables of the 60-bit fixed-point kernel (sfmm_tables.hpp, FxTables),
-// one set per group size; the edge factors (e_in_M, e_in_L, e_out_L, e_out_M)
-// are shared by the sets
+// device tables of the 60-bit fixed-point or the FP32 kernel (sfmm_tables.hpp,
+// FxTables and F32Tables), one set per group size; the edge factors (e_in_M,
+// e_in_L, e_out_L, e_out_M) are shared by the sets
 struct FxDevTables {
     void *W = nullptr, *H[3] = {nullptr, nullptr, nullptr};
     int *woff = nullptr, *hoff = nullptr;
@@ -95,7 +95,7 @@ struct sfmm_context {
     cudaStream_t stream = nullptr;
     sfmm::HostTables host;
     sfmm::DevTables tab[sfmm::kNumArith];  // indexed by Arith (the tensor-core modes use tc[])
-    sfmm::FxDevTables fxt[2];  // 4 and 8 threads per translation
+    sfmm::FxDevTables fxt[2], f32t[2];  // 4 and 8 threads per translation
     void *fx_edge[4] = {nullptr, nullptr, nullptr, nullptr};
     sfmm::TcDevTables *tc[3] = {nullptr, nullptr, nullptr};  // tensor-core operand images by format
     std::string err;

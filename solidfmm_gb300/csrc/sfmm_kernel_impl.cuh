@@ -84,47 +84,60 @@ static int occupancy_typed(const LaunchShape &s)
     return 0;
 }
 
-template <int G, int ACC>
+template <class A, int G, int ACC>
 static cudaError_t launch_fx_inst(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
 {
     clear_stale_error();
     if (p.work) {
         if (!p.in_hbm) return cudaErrorInvalidValue;  // work lists are a device-memory form
-        k_translate_fx<G, ACC, true, true><<<grid, s.threads, s.smem, st>>>(p);
+        k_translate_fx<A, G, ACC, true, true><<<grid, s.threads, s.smem, st>>>(p);
     } else if (p.in_hbm) {
-        k_translate_fx<G, ACC, true><<<grid, s.threads, s.smem, st>>>(p);
+        k_translate_fx<A, G, ACC, true><<<grid, s.threads, s.smem, st>>>(p);
     } else {
-        k_translate_fx<G, ACC, false><<<grid, s.threads, s.smem, st>>>(p);
+        k_translate_fx<A, G, ACC, false><<<grid, s.threads, s.smem, st>>>(p);
     }
     return cudaGetLastError();
 }
 
-template <int G, int ACC>
+template <class A, int G, int ACC>
 static int occupancy_fx_inst(const LaunchShape &s)
 {
-    auto kern = k_translate_fx<G, ACC>;
+    auto kern = k_translate_fx<A, G, ACC>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    cudaFuncSetAttribute(k_translate_fx<G, ACC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-    cudaFuncSetAttribute(k_translate_fx<G, ACC, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    cudaFuncSetAttribute(k_translate_fx<A, G, ACC, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+    cudaFuncSetAttribute(k_translate_fx<A, G, ACC, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, s.threads, s.smem) != cudaSuccess) return 0;
     return nb;
 }
 
-static inline cudaError_t launch_fx(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
+// FP64: row blocks by the registers of a full SM; FP32 (orders up to 28): two sizes
+#define SFMM_FOR_F32_SHAPES(X) X(4, 4) X(4, 6) X(4, 8) X(4, 10) X(4, 14) X(8, 4) X(8, 6) X(8, 8)
+
+template <class A>
+static cudaError_t launch_fx(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
 {
 #define X(G_, A_) \
-    if (s.G == G_ && s.acc == A_) return launch_fx_inst<G_, A_>(p, s, grid, st);
-    SFMM_FOR_FX_SHAPES(X)
+    if (s.G == G_ && s.acc == A_) return launch_fx_inst<A, G_, A_>(p, s, grid, st);
+    if constexpr (std::is_same<A, float>::value) {
+        SFMM_FOR_F32_SHAPES(X)
+    } else {
+        SFMM_FOR_FX_SHAPES(X)
+    }
 #undef X
     return cudaErrorInvalidValue;
 }
 
-static inline int occupancy_fx(const LaunchShape &s)
+template <class A>
+static int occupancy_fx(const LaunchShape &s)
 {
 #define X(G_, A_) \
-    if (s.G == G_ && s.acc == A_) return occupancy_fx_inst<G_, A_>(s);
-    SFMM_FOR_FX_SHAPES(X)
+    if (s.G == G_ && s.acc == A_) return occupancy_fx_inst<A, G_, A_>(s);
+    if constexpr (std::is_same<A, float>::value) {
+        SFMM_FOR_F32_SHAPES(X)
+    } else {
+        SFMM_FOR_FX_SHAPES(X)
+    }
 #undef X
     return 0;
 }

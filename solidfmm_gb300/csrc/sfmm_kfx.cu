@@ -4,7 +4,7 @@
 namespace sfmm {
 cudaError_t launch_translate_fx(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
 {
-    return launch_fx(p, s, grid, st);
+    return launch_fx<double>(p, s, grid, st);
 }
-int occupancy_fx64(const LaunchShape &s) { return occupancy_fx(s); }
+int occupancy_fx64(const LaunchShape &s) { return occupancy_fx<double>(s); }
 }  // namespace sfmm

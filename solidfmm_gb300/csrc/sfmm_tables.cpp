@@ -218,6 +218,47 @@ FxTables build_fx_tables(const HostTables &t, int G, int P)
     return f;
 }
 
+F32Tables build_f32_tables(const HostTables &t, int G, int P)
+{
+    F32Tables f;
+    const int RS = G / 2;
+    f.woff.resize(P);
+    size_t tot = 0;
+    for (int n = 0; n < P; ++n) {
+        f.woff[n] = (int)tot;
+        tot += size_t((n + 2) / 2) * (((n + RS) / RS + 3) / 4) * 4 * G;
+    }
+    f.W.assign(tot, 0.f);
+    for (int n = 0; n < P; ++n) {
+        const int d = n + 1, NA = (d + RS - 1) / RS, slot = (NA + 3) / 4 * 4 * G;
+        for (int tt = 0; tt < (d + 1) / 2; ++tt)
+            for (int q = 0; q < G; ++q)
+                for (int a = 0; a < NA; ++a) {
+                    const int part = q & 1, i = (q >> 1) + RS * a, j = ((i + n + part) & 1) + 2 * tt;
+                    f.W[f.woff[n] + size_t(tt) * slot + a / 4 * 4 * G + 4 * q + a % 4] = (float)w_entry(t, n, part, i, j);
+                }
+    }
+    f.hoff.resize(P);
+    tot = 0;
+    for (int m = 0; m < P; ++m) {
+        f.hoff[m] = (int)tot;
+        tot += size_t(P - m) * fx_hrow(P - m, G, 4);
+    }
+    for (int op = 0; op < 3; ++op) {
+        f.H[op].assign(tot, 0.f);
+        for (int m = 0; m < P; ++m) {
+            const int HR = hrows(t.P - m, t.pad), hs = fx_hrow(P - m, G, 4);
+            for (int k = 0; k < P - m; ++k)
+                for (int np = 0; np < P - m; ++np) {
+                    const int r = np % RS, b = np / RS;
+                    f.H[op][f.hoff[m] + size_t(k) * hs + b / 4 * 2 * G + 4 * r + b % 4] =
+                        (float)t.H[op][t.hoff[m] + size_t(k) * HR + np];
+                }
+        }
+    }
+    return f;
+}
+
 std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count)
 {
     std::vector<int32_t> out(4 * count);

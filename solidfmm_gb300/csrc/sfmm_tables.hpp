@@ -93,6 +93,15 @@ struct FxTables {
     std::vector<int> hoff;
 };
 FxTables build_fx_tables(const HostTables &t, int G, int P);
+// The same tables for the FP32 kernel: swap coefficients in FP32, degree n at
+// woff[n], slot t 4 NQ G further (NQ = ceil(NA / 4)), lane q's rows a at
+// (a / 4) 4 G + 4 q + a % 4; z matrices in FP32, output n' at
+// (b / 4) 2 G + 4 r + b % 4 of a row of fx_hrow(P - m, G, 4) elements.
+struct F32Tables {
+    std::vector<float> W, H[3];
+    std::vector<int> woff, hoff;
+};
+F32Tables build_f32_tables(const HostTables &t, int G, int P);
 // positive edge factors as (h, l, exponent, 0): (h 2^30 + l) 2^(exponent - 60)
 std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count);
 

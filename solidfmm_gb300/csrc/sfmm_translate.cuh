@@ -35,6 +35,7 @@
 
 #include "sfmm_arith.cuh"
 #include "sfmm_fixed.cuh"
+#include "sfmm_f32.cuh"
 #include "sfmm_fx.cuh"
 #include "sfmm_params.hpp"
 
@@ -84,6 +85,27 @@ __device__ __forceinline__ void dispatch(int na, F &&f)
     case 8: if constexpr (MAXN >= 8) f(ic<8>{}); break;
     default: break;
     }
+}
+
+// f(ic<NA>, n) for the degrees n < count in order, NA = ceil((n + 1) / RS):
+// RS degrees in a row share an instance, so that no degree pays for a switch.
+template <int MAXN, int RS, int NA = 1, class F>
+__device__ __forceinline__ void for_degrees(int count, F &&f)
+{
+#pragma unroll 1
+    for (int n = RS * (NA - 1); n < min(RS * NA, count); ++n) f(ic<NA>{}, n);
+    if constexpr (NA < MAXN)
+        if (RS * NA < count) for_degrees<MAXN, RS, NA + 1>(count, f);
+}
+
+// f(ic<NB>, m) for the columns m < mend in order, NB = ceil((nout - m) / RS)
+template <int NB, int RS, class F>
+__device__ __forceinline__ void for_columns(int m, int mend, int nout, F &&f)
+{
+#pragma unroll 1
+    for (; m < mend && nout - m > RS * (NB - 1); ++m) f(ic<NB>{}, m);
+    if constexpr (NB > 1)
+        if (m < mend) for_columns<NB - 1, RS>(m, mend, nout, f);
 }
 
 // Rows of a degree's swap-coefficient block in the instance that runs NA
@@ -609,15 +631,17 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     using Src = typename src_of<A>::type;
     static_assert(sizeof(S) == sizeof(Src), "buffer slots hold one source value");
     static_assert(32 % G == 0, "a translation's threads must share a warp");
-    // block fixed point: 30-bit mantissas in the float-float kernel, 60-bit in FP64
-    constexpr bool FX = FIX && std::is_same<A, double>::value;
-    static_assert(!FIX || AR::split || FX, "fixed-point swaps are a float-float or FP64 variant");
+    // FIX: the float-float kernel with 30-bit block fixed-point swaps, or the
+    // kernels whose lanes hold one part of an element each (PL): FP64 in
+    // 60-bit block fixed point, and FP32
+    constexpr bool PL = FIX && !AR::split;
+    constexpr bool F32 = std::is_same<A, float>::value;
 
     // Loads in flight per lane in the source gather and the target update,
     // measured on GB300 (M2L P=16, 10^6): 8 and 4 make the split kernel 2.2%
     // and the FP32 kernel 3.7% faster than 4 and 1, which the FP64 and
     // float-float kernels keep (1.5% and 0.7% slower with 8 and 4).
-    constexpr bool kDeep = FIX || std::is_same<A, float>::value;
+    constexpr bool kDeep = FIX;
     // FP32-range arithmetics run every translation at the length scale of
     // its shift: lambda = 2^ks with |shift| / lambda in [2, 7), sources (and
     // the shift) divided by lambda^n (multipoles) or lambda^-(n+1) (locals),
@@ -628,7 +652,7 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     // inside the FP32 range at every geometry scale; shifts whose largest
     // component lies in [2, 4) run unscaled
     constexpr bool kScale = !std::is_same<A, double>::value;
-    constexpr int kGatherUnroll = kDeep || FX ? 8 : 4;
+    constexpr int kGatherUnroll = kDeep ? 8 : 4;
     constexpr int kAccUnroll = kDeep ? 4 : 1;
     constexpr int kAccBatch = 5;
 
@@ -644,8 +668,8 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     const unsigned FULL = 0xffffffffu;
 
     S *buf0 = reinterpret_cast<S *>(smem);
-    FxGeo *geo = reinterpret_cast<FxGeo *>(smem + (size_t)TS * p.spad * sizeof(S));  // FX only
-    uint32_t *meta = reinterpret_cast<uint32_t *>(smem + (size_t)TS * p.spad * sizeof(S) + (FX ? TS * sizeof(FxGeo) : 0));
+    FxGeo *geo = reinterpret_cast<FxGeo *>(smem + (size_t)TS * p.spad * sizeof(S));  // PL only
+    uint32_t *meta = reinterpret_cast<uint32_t *>(smem + (size_t)TS * p.spad * sizeof(S) + (PL ? TS * sizeof(FxGeo) : 0));
     uint32_t *m_sidx = meta;
     uint32_t *m_tidx = meta + TS;
     uint32_t *m_pin = meta + 2 * TS;
@@ -659,13 +683,13 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     const Src *src = reinterpret_cast<const Src *>(p.src);
     Src *dst = reinterpret_cast<Src *>(p.dst);
     const int op = p.op;
-    if constexpr (FX) {
+    if constexpr (PL) {
         // this order's tables into L1, all loads in flight at once (the
         // transforms would meet them one miss after the other)
         touch_tables(p.W, p.wbytes);
         touch_tables(p.H, p.hbytes);
-        touch_tables(p.ein, P * (P + 1) / 2 * 16);
-        touch_tables(p.eout, P * (P + 1) / 2 * 16);
+        touch_tables(p.ein, P * (P + 1) / 2 * (F32 ? 4 : 16));
+        touch_tables(p.eout, P * (P + 1) / 2 * (F32 ? 4 : 16));
     }
 
     for (long long tile = blockIdx.x;; tile += gridDim.x) {
@@ -746,10 +770,10 @@ __device__ __forceinline__ void translate_body(const KParams &p)
             m_pin[slot] = (uint32_t)pin | ((uint32_t)(ks + 32768) << 16);  // order, and the scale above it
             m_pout[slot] = pout;
             m_id[slot] = ident_p;
-            if constexpr (FX) *reinterpret_cast<double3 *>(geo + slot) = make_double3(x, y, z);
+            if constexpr (PL) *reinterpret_cast<double3 *>(geo + slot) = make_double3(x, y, z);
         }
         __syncthreads();
-        if constexpr (FX) {  // one thread per translation: the others' lanes would only repeat it
+        if constexpr (PL) {  // one thread per translation: the others' lanes would only repeat it
             if (tid < TS) {
                 const double3 v = *reinterpret_cast<const double3 *>(geo + tid);
                 fx_geometry(v.x, v.y, v.z, geo + tid);
@@ -772,6 +796,16 @@ __device__ __forceinline__ void translate_body(const KParams &p)
                 const int ksg = (int)(m_pin[s] >> 16) - 32768;
                 const int es = op == OP_L2L ? ksg : -ksg;  // per degree
                 const int e0 = op == OP_L2L ? ksg : 0;
+                if constexpr (F32) {
+                    // every factor an FP32 normal: plain products (a result
+                    // below the normal range keeps what digits it has)
+                    if (abs(es) * P + abs(e0) <= 126) {
+#pragma unroll(kGatherUnroll)
+                        for (int c = lane; c < p.spad; c += 32)
+                            bp[c] = c < cnt ? __ldcs(sp + c) * pow2f(es * degree_at(c) + e0) : 0.f;
+                        continue;
+                    }
+                }
 #pragma unroll(kGatherUnroll)
                 for (int c = lane; c < p.spad; c += 32)
                     AR::st(bp + c, c < cnt ? src_scaled(__ldcs(sp + c), es * degree_at(c) + e0, (const T *)nullptr)
@@ -816,7 +850,61 @@ __device__ __forceinline__ void translate_body(const KParams &p)
         const int pin_w = __reduce_max_sync(FULL, pin);
         const int pout_w = __reduce_max_sync(FULL, pout);
 
-        if constexpr (FX) {
+        if constexpr (PL && F32) {
+            const FxGeo &ge = geo[slot];
+            const int part = q & 1;
+            F32Trig<ACC> tg;
+            {
+                fx c[ACC], sn[ACC];
+                fx_powers<G / 2, ACC>(ge.ca, ge.sa, q >> 1, part, c, sn);
+#pragma unroll
+                for (int a = 0; a < ACC; ++a) {
+                    tg.ca[a] = f32_of_fx(c[a]);
+                    tg.sa[a] = f32_of_fx(sn[a]);
+                }
+                fx_powers<G / 2, ACC>(ge.cb, ge.sb, q >> 1, part, c, sn);
+#pragma unroll
+                for (int a = 0; a < ACC; ++a) {
+                    tg.cb[a] = f32_of_fx(c[a]);
+                    tg.sb[a] = f32_of_fx(sn[a]);
+                }
+            }
+            // the scaled |shift| lies in [2, 7); not finite or zero: NaN
+            const bool bad = ge.re == kFxBad;
+            const ff nan{__int_as_float(0x7fffffff), 0.f}, one{1.f, 0.f};
+            const ff r = bad ? nan : ff_of_fxs(ge.r, ge.re), rinv = bad ? nan : ff_of_fxs(ge.rinv, ge.rinve);
+            // 2. forward transforms: r^n (L input) or r^-(n+1) (M input)
+            ff f = op == OP_L2L ? (bad ? nan : one) : rinv;
+            const ff fstep = op == OP_L2L ? r : rinv;
+            const T *w = W, *e = EIN;
+            for_degrees<ACC, G / 2>(pin_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                forward_degree_f32<G, NA, ACC>(b, n, w, e, f.hi, q, tg);
+                w += ((n + 2) >> 1) * ((NA + 3) / 4 * 4 * G);
+                e += n + 1;
+                f = ff_mul(f, fstep);
+            });
+            // 3. z-translation (columns m >= min(P_in, P_out) of the outputs
+            // stay zero: their rows beyond P_in were zero-filled by the gather)
+            const T *h = H;
+            for_columns<ACC, G / 2>(0, min(pin_w, pout_w), pout_w, [&](auto nb, int m) {
+                const int hs = fx_hrow(p.Ptab - m, G, 4);
+                z_column_part<float, G, decltype(nb)::value>(b, h, hs, m, op == OP_M2M ? min(pin_w, pout_w) : pin_w, pout_w, q);
+                h += (p.Ptab - m) * hs;
+            });
+            // 4. backward transforms: r^(n+1) (M output) or r^-n (L output)
+            f = op == OP_M2M ? r : one;
+            const ff bstep = op == OP_M2M ? r : rinv;
+            w = W;
+            e = EOUT;
+            for_degrees<ACC, G / 2>(pout_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                backward_degree_f32<G, NA, ACC>(b, n, w, e, f.hi, q, tg);
+                w += ((n + 2) >> 1) * ((NA + 3) / 4 * 4 * G);
+                e += n + 1;
+                f = ff_mul(f, bstep);
+            });
+        } else if constexpr (PL) {
             const FxGeo &ge = geo[slot];
             const int part = q & 1;
             FxTrig<ACC> tg;
@@ -829,30 +917,36 @@ __device__ __forceinline__ void translate_body(const KParams &p)
             const double *H = reinterpret_cast<const double *>(p.H);
             // 2. forward transforms: r^n (L input) or r^-(n+1) (M input)
             fxs f = op == OP_L2L ? one : rinv;
-            for (int n = 0; n < pin_w; ++n) {
-                dispatch<ACC>((n + G / 2) / (G / 2), [&](auto na) {
-                    forward_degree_fx<G, decltype(na)::value, ACC>(b, n, W + __ldg(p.woff + n), EIN + n * (n + 1) / 2, f,
-                                                                  bad, q, tg);
-                });
-                f = fxs_mul(f, op == OP_L2L ? r : rinv);
-            }
+            const fxs fstep = op == OP_L2L ? r : rinv;
+            const int2 *w = W;
+            const int4 *e = EIN;
+            for_degrees<ACC, G / 2>(pin_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                forward_degree_fx<G, NA, ACC>(b, n, w, e, f, bad, q, tg);
+                w += ((n + 2) >> 1) * (NA * G);
+                e += n + 1;
+                f = fxs_mul(f, fstep);
+            });
             // 3. z-translation (columns m >= min(P_in, P_out) of the outputs
             // stay zero: their rows beyond P_in were zero-filled by the gather)
-            const int mend = min(pin_w, pout_w);
-            for (int m = 0; m < mend; ++m)
-                dispatch<ACC>((pout_w - m + G / 2 - 1) / (G / 2), [&](auto nb) {
-                    z_column_op<double, G, decltype(nb)::value>(op, b, H + __ldg(p.hoff + m), fx_hrow(p.Ptab - m, G), m,
-                                                                pin_w, pout_w, q);
-                });
+            const double *h = H;
+            for_columns<ACC, G / 2>(0, min(pin_w, pout_w), pout_w, [&](auto nb, int m) {
+                const int hs = fx_hrow(p.Ptab - m, G);
+                z_column_op<double, G, decltype(nb)::value>(op, b, h, hs, m, pin_w, pout_w, q);
+                h += (p.Ptab - m) * hs;
+            });
             // 4. backward transforms: r^(n+1) (M output) or r^-n (L output)
             f = op == OP_M2M ? r : one;
-            for (int n = 0; n < pout_w; ++n) {
-                dispatch<ACC>((n + G / 2) / (G / 2), [&](auto na) {
-                    backward_degree_fx<G, decltype(na)::value, ACC>(b, n, W + __ldg(p.woff + n), EOUT + n * (n + 1) / 2,
-                                                                   f, bad, q, tg);
-                });
-                f = fxs_mul(f, op == OP_M2M ? r : rinv);
-            }
+            const fxs bstep = op == OP_M2M ? r : rinv;
+            w = W;
+            e = EOUT;
+            for_degrees<ACC, G / 2>(pout_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                backward_degree_fx<G, NA, ACC>(b, n, w, e, f, bad, q, tg);
+                w += ((n + 2) >> 1) * (NA * G);
+                e += n + 1;
+                f = fxs_mul(f, bstep);
+            });
         } else {
             // geometry (euler, microkernel_generic.cpp:37-97)
             Geometry<AR, G, ACC, FIX> geo(x, y, z, q);
@@ -944,7 +1038,27 @@ __device__ __forceinline__ void translate_body(const KParams &p)
             // degree j times lambda^j (multipoles) or lambda^-(j+1) (locals)
             const int ksa = (int)(m_pin[s] >> 16) - 32768;
             const int eo = op == OP_M2M ? ksa : -ksa, eo0 = op == OP_M2M ? 0 : -ksa;
-            if constexpr (FX) {
+            if constexpr (PL && F32) {
+                // the FP32 sum equals the FP64 sum rounded to FP32
+                if (!pid && abs(eo) * P + abs(eo0) <= 126) {
+                    for (int c0 = lane; c0 < cnt; c0 += 32 * kAccBatch) {
+                        float v[kAccBatch];
+                        if (!p.atomic) {
+#pragma unroll
+                            for (int u = 0; u < kAccBatch; ++u) v[u] = c0 + 32 * u < cnt ? __ldcs(dp + c0 + 32 * u) : 0.f;
+                        }
+#pragma unroll
+                        for (int u = 0; u < kAccBatch; ++u) {
+                            const int c = c0 + 32 * u;
+                            if (c >= cnt) continue;
+                            const float y = bp[c] * pow2f(eo * degree_at(c) + eo0);
+                            if (p.atomic) atomicAdd(dp + c, y);
+                            else __stcs(dp + c, v[u] + y);
+                        }
+                    }
+                    continue;
+                }
+            } else if constexpr (PL) {
                 // kAccBatch target loads in flight per lane
                 if (!p.atomic && !pid) {
                     for (int c0 = lane; c0 < cnt; c0 += 32 * kAccBatch) {
@@ -998,12 +1112,18 @@ __global__ void __launch_bounds__(256) k_translate(KParams p)
     translate_body<A, G, ACC, FIX, HBM, WORK>(p);
 }
 
-constexpr int fx_blocks(int acc) { return acc <= 4 ? 5 : acc <= 6 ? 4 : 2; }
-// FP64 in 60-bit block fixed point
-template <int G, int ACC, bool HBM = true, bool WORK = false>
-__global__ void __launch_bounds__(kFxThreads, fx_blocks(ACC)) k_translate_fx(KParams p)
+// resident CTAs per SM that the registers have to allow
+template <class A>
+constexpr int fx_blocks(int acc)
 {
-    translate_body<double, G, ACC, true, HBM, WORK>(p);
+    if (std::is_same<A, float>::value) return acc <= 4 ? 8 : acc <= 6 ? 6 : acc <= 8 ? 5 : acc <= 10 ? 4 : 2;
+    return acc <= 4 ? 5 : acc <= 6 ? 4 : 2;
+}
+// FP64 in 60-bit block fixed point (A = double), FP32 (A = float)
+template <class A, int G, int ACC, bool HBM = true, bool WORK = false>
+__global__ void __launch_bounds__(kFxThreads, fx_blocks<A>(ACC)) k_translate_fx(KParams p)
+{
+    translate_body<A, G, ACC, true, HBM, WORK>(p);
 }
 
 }  // namespace sfmm
