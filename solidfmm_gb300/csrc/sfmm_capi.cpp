@@ -48,34 +48,17 @@ int cuda_fail(sfmm_context *c, cudaError_t e, const char *what)
 
 size_t esize(Arith a) { return a == Arith::F32 ? sizeof(float) : (a == Arith::F64 ? sizeof(double) : 2 * sizeof(float)); }
 
-// convert an FP64 table into the arithmetic's element type
-std::vector<unsigned char> convert(const std::vector<double> &v, Arith a)
+namespace {
+
+template <class T>
+cudaError_t put(void **dst, const std::vector<T> &v)
 {
-    std::vector<unsigned char> out(v.size() * esize(a));
-    for (size_t i = 0; i < v.size(); ++i) {
-        if (a == Arith::F64) {
-            std::memcpy(&out[i * 8], &v[i], 8);
-        } else if (a == Arith::F32) {
-            float f = (float)v[i];
-            std::memcpy(&out[i * 4], &f, 4);
-        } else {
-            float hi = (float)v[i];
-            float lo = (float)(v[i] - (double)hi);
-            std::memcpy(&out[i * 8], &hi, 4);
-            std::memcpy(&out[i * 8 + 4], &lo, 4);
-        }
-    }
-    return out;
+    cudaError_t e = cudaMalloc(dst, v.empty() ? 16 : v.size() * sizeof(T));
+    if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+    return e;
 }
 
-cudaError_t upload(void **dst, const std::vector<double> &v, Arith a)
-{
-    auto bytes = convert(v, a);
-    cudaError_t e = cudaMalloc(dst, bytes.size() ? bytes.size() : 16);
-    if (e != cudaSuccess) return e;
-    if (bytes.empty()) return cudaSuccess;
-    return cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
-}
+}  // namespace
 
 void free_fx(FxDevTables &t)
 {
@@ -87,7 +70,7 @@ void free_fx(FxDevTables &t)
 
 void free_tables(DevTables &t)
 {
-    void *ps[] = {t.W, t.ein_M, t.ein_L, t.eout_L, t.eout_M, t.H[0], t.H[1], t.H[2], t.Wq, t.W8, t.Wq8};
+    void *ps[] = {t.W, t.ein_M, t.ein_L, t.eout_L, t.eout_M, t.H[0], t.H[1], t.H[2]};
     for (void *p : ps)
         if (p) cudaFree(p);
     t = DevTables{};
@@ -97,34 +80,15 @@ namespace {
 
 void free_offsets(sfmm_context *c)
 {
-    int **ps[] = {&c->d_woff, &c->d_hoff, &c->d_woff8};
-    for (int **p : ps) {
+    for (int **p : {&c->d_woff, &c->d_hoff}) {
         if (*p) cudaFree(*p);
         *p = nullptr;
     }
 }
 
-// the offset arrays of the tables, all or none (a partial set is freed)
-cudaError_t upload_offsets(sfmm_context *c)
-{
-    const size_t n8 = c->host.woff8.size();
-    if (c->d_woff && c->d_hoff && (!n8 || c->d_woff8)) return cudaSuccess;
-    free_offsets(c);
-    cudaError_t e = cudaMalloc(&c->d_woff, sizeof(int) * c->P);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_hoff, sizeof(int) * c->P);
-    if (e == cudaSuccess && n8) e = cudaMalloc(&c->d_woff8, sizeof(int) * n8);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(c->d_woff, c->host.woff.data(), sizeof(int) * c->P, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(c->d_hoff, c->host.hoff.data(), sizeof(int) * c->P, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && n8)
-        e = cudaMemcpy(c->d_woff8, c->host.woff8.data(), sizeof(int) * n8, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) free_offsets(c);
-    return e;
-}
-
 }  // namespace
 
+// tables of a tensor-core arithmetic, or of FP64 above order 32, once per context
 int ensure_tables(sfmm_context *c, Arith a)
 {
     if (is_tc(a)) {
@@ -134,54 +98,35 @@ int ensure_tables(sfmm_context *c, Arith a)
         if (e != cudaSuccess) return cuda_fail(c, e, "tensor-core table upload");
         return SFMM_OK;
     }
-    DevTables &t = c->tab[(int)a];
+    DevTables &t = c->tab;
     if (t.ready) return SFMM_OK;
-    cudaError_t e = upload_offsets(c);
-    if (e != cudaSuccess) return cuda_fail(c, e, "table upload");
-    const bool w8 = !c->host.W8.empty();
-    // |w| <= 1 (orthogonal matrices): round(w 2^30) fits int32
-    auto upload_q30 = [](void **dst, const std::vector<double> &W) {
-        std::vector<int32_t> q(W.size());
-        for (size_t i = 0; i < q.size(); ++i) q[i] = (int32_t)std::llround(std::ldexp(W[i], 30));
-        cudaError_t err = cudaMalloc(dst, q.size() * sizeof(int32_t) + 16);
-        if (err == cudaSuccess) err = cudaMemcpy(*dst, q.data(), q.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-        return err;
-    };
-    e = upload(&t.W, c->host.W, a);
-    if (e == cudaSuccess && w8) e = upload(&t.W8, c->host.W8, a);
-    if (e == cudaSuccess) e = upload(&t.ein_M, c->host.e_in_M, a);
-    if (e == cudaSuccess) e = upload(&t.ein_L, c->host.e_in_L, a);
-    if (e == cudaSuccess) e = upload(&t.eout_L, c->host.e_out_L, a);
-    if (e == cudaSuccess) e = upload(&t.eout_M, c->host.e_out_M, a);
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = upload(&t.H[k], c->host.H[k], a);
-    if (e == cudaSuccess && a == Arith::FFQ) e = upload_q30(&t.Wq, c->host.W);
-    if (e == cudaSuccess && a == Arith::FFQ && w8) e = upload_q30(&t.Wq8, c->host.W8);
+    cudaError_t e = put((void **)&c->d_woff, c->host.woff);
+    if (e == cudaSuccess) e = put((void **)&c->d_hoff, c->host.hoff);
+    if (e == cudaSuccess) e = put(&t.W, c->host.W);
+    if (e == cudaSuccess) e = put(&t.ein_M, c->host.e_in_M);
+    if (e == cudaSuccess) e = put(&t.ein_L, c->host.e_in_L);
+    if (e == cudaSuccess) e = put(&t.eout_L, c->host.e_out_L);
+    if (e == cudaSuccess) e = put(&t.eout_M, c->host.e_out_M);
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], c->host.H[k]);
     if (e != cudaSuccess) {
         free_tables(t);  // a partial set is retried from scratch on the next call
+        free_offsets(c);
         return cuda_fail(c, e, "table upload");
     }
     t.ready = true;
     return SFMM_OK;
 }
 
-
 namespace {
-
-cudaError_t put(void **dst, const void *src, size_t bytes)
-{
-    cudaError_t e = cudaMalloc(dst, bytes);
-    if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
-    return e;
-}
 
 // the tables of one group size: swap coefficients of wsize bytes per woff unit
 template <class T>
 cudaError_t put_fx(FxDevTables &t, const T &h, int P, size_t wsize)
 {
-    cudaError_t e = put(&t.W, h.W.data(), h.W.size() * sizeof(h.W[0]));
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k].data(), h.H[k].size() * sizeof(h.H[k][0]));
-    if (e == cudaSuccess) e = put((void **)&t.woff, h.woff.data(), h.woff.size() * sizeof(int));
-    if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff.data(), h.hoff.size() * sizeof(int));
+    cudaError_t e = put(&t.W, h.W);
+    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k]);
+    if (e == cudaSuccess) e = put((void **)&t.woff, h.woff);
+    if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff);
     t.wend.assign(P + 1, (int)(h.W.size() * sizeof(h.W[0])));
     for (int n = 0; n < P; ++n) t.wend[n] = (int)(h.woff[n] * wsize);
     t.hbytes = (int)(h.H[0].size() * sizeof(h.H[0][0]));
@@ -189,36 +134,43 @@ cudaError_t put_fx(FxDevTables &t, const T &h, int P, size_t wsize)
     return e;
 }
 
+// edge factors in the arithmetic's form
+cudaError_t put_edges(void **dst, Arith a, const std::vector<double> &e, size_t ne)
+{
+    if (a == Arith::F64) return put(dst, fx_edges(e, ne));
+    std::vector<float> v;
+    for (size_t i = 0; i < ne; ++i) {
+        v.push_back((float)e[i]);
+        if (a == Arith::FFQ) v.push_back((float)(e[i] - (double)v.back()));
+    }
+    return put(dst, v);
+}
+
 }  // namespace
 
-// Tables of the 60-bit fixed-point kernel (FP64) or of the FP32 kernel for G
-// threads per translation (orders up to 32), once per context.
+// Tables of the 60-bit fixed-point (F64), the FP32 or the split kernel (FFQ)
+// for G threads per translation (orders up to 32), once per context.
 int ensure_fx(sfmm_context *c, Arith a, int G)
 {
-    FxDevTables &t = (a == Arith::F32 ? c->f32t : c->fxt)[G == 8];
+    FxDevTables &t = c->fxt[(int)a][G == 8];
     if (t.ready) return SFMM_OK;
     const int P = std::min(c->P, 32);
     cudaError_t e = cudaSuccess;
     try {
         const std::vector<double> *ev[4] = {&c->host.e_in_M, &c->host.e_in_L, &c->host.e_out_L, &c->host.e_out_M};
-        const size_t ne = (size_t)P * (P + 1) / 2;
         for (int k = 0; k < 4 && e == cudaSuccess; ++k) {
-            if (c->fx_edge[k]) continue;  // a context has one data type
-            if (a == Arith::F32) {
-                const std::vector<float> v(ev[k]->begin(), ev[k]->begin() + ne);
-                e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(float));
-            } else {
-                const auto v = fx_edges(*ev[k], ne);
-                e = put(&c->fx_edge[k], v.data(), v.size() * sizeof(int32_t));
-            }
-            if (e != cudaSuccess && c->fx_edge[k]) {
-                cudaFree(c->fx_edge[k]);
-                c->fx_edge[k] = nullptr;
+            void *&d = c->fx_edge[(int)a][k];
+            if (d) continue;
+            e = put_edges(&d, a, *ev[k], (size_t)P * (P + 1) / 2);
+            if (e != cudaSuccess && d) {
+                cudaFree(d);
+                d = nullptr;
             }
         }
         if (e == cudaSuccess)
-            e = a == Arith::F32 ? put_fx(t, build_f32_tables(c->host, G, P), P, sizeof(float))
-                                : put_fx(t, build_fx_tables(c->host, G, P), P, 2 * sizeof(int32_t));
+            e = a == Arith::F32   ? put_fx(t, build_f32_tables(c->host, G, P), P, sizeof(float))
+                : a == Arith::F64 ? put_fx(t, build_fx_tables(c->host, G, P), P, 2 * sizeof(int32_t))
+                                  : put_fx(t, build_split_tables(c->host, G, P), P, 2 * sizeof(int32_t));
     } catch (const std::bad_alloc &) {
         free_fx(t);
         return fail(c, SFMM_OOM, "operator tables");
@@ -383,24 +335,20 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
         return SFMM_OK;
     }
     if (s.fx) {
-        const FxDevTables &t = (a == Arith::F32 ? c->f32t : c->fxt)[s.G == 8];
+        const FxDevTables &t = c->fxt[(int)a][s.G == 8];
         p.W = t.W;
         p.woff = t.woff;
         p.hoff = t.hoff;
         p.Ptab = t.P;
-        p.ein = c->fx_edge[op == SFMM_L2L ? 1 : 0];
-        p.eout = c->fx_edge[op == SFMM_M2M ? 3 : 2];
+        p.ein = c->fx_edge[(int)a][op == SFMM_L2L ? 1 : 0];
+        p.eout = c->fx_edge[(int)a][op == SFMM_M2M ? 3 : 2];
         p.H = t.H[op];
         p.wbytes = t.wend[Pbound];
         p.hbytes = t.P == Pbound ? t.hbytes : 0;  // a smaller bound reads parts of every row
     } else {
-        const DevTables &t = c->tab[(int)a];
-        // swap blocks padded for this launch's group size (4 or 8 threads per
-        // translation step 8 rows, one warp 32)
-        const bool w8 = s.G != 32 && c->d_woff8;
-        p.W = w8 ? t.W8 : t.W;
-        p.Wq = static_cast<const int *>(w8 ? t.Wq8 : t.Wq);
-        p.woff = w8 ? c->d_woff8 : c->d_woff;
+        const DevTables &t = c->tab;
+        p.W = t.W;
+        p.woff = c->d_woff;
         p.hoff = c->d_hoff;
         p.rowpad = c->host.pad;
         p.ein = (op == SFMM_L2L) ? t.ein_L : t.ein_M;
@@ -441,20 +389,24 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     int acc = (P + G - 1) / G;
     if (G == 4) acc = acc <= 2 ? 2 : (acc <= 4 ? 4 : (acc <= 6 ? 6 : 8));
     if (G == 32) acc = acc <= 2 ? 2 : 3;
-    // FP64 (in 60-bit fixed point) and FP32 up to order 32: rows in steps of
-    // G/2; four threads per translation only up to order 16 (more rows than
-    // their registers hold: above, a request for 4 runs 8)
-    s.fx = (a == Arith::F64 || a == Arith::F32) && G != 32;
-    if (s.fx) {
-        if (P > 16 && G == 4 && a == Arith::F64) {
-            G = 8;
-            ts /= 2;
-            if (ts < 32 / G || ts % (32 / G)) return s;
+    s.fx = G != 32;
+    if (a == Arith::F64 || a == Arith::F32) {
+        // one part of an element per lane, rows in steps of G/2.  FP64 runs
+        // four threads per translation only up to order 16 (more rows than
+        // their registers hold: above, a request for 4 runs 8)
+        if (G != 32) {
+            if (P > 16 && G == 4 && a == Arith::F64) {
+                G = 8;
+                ts /= 2;
+                if (ts < 32 / G || ts % (32 / G)) return LaunchShape{};
+            }
+            if (G * ts > kFxThreads) return LaunchShape{};
+            acc = (P + G / 2 - 1) / (G / 2);
+            if (a == Arith::F32) acc = acc <= 4 ? 4 : acc <= 6 ? 6 : acc <= 8 ? 8 : acc <= 10 ? 10 : 14;
+            else acc = G == 4 ? (acc <= 4 ? 4 : acc <= 6 ? 6 : 8) : (acc + 1) / 2 * 2;
         }
-        if (G * ts > kFxThreads) return LaunchShape{};
-        acc = (P + G / 2 - 1) / (G / 2);
-        if (a == Arith::F32) acc = acc <= 4 ? 4 : acc <= 6 ? 6 : acc <= 8 ? 8 : acc <= 10 ? 10 : 14;
-        else acc = G == 4 ? (acc <= 4 ? 4 : acc <= 6 ? 6 : 8) : (acc + 1) / 2 * 2;
+    } else if (G == 32) {
+        return LaunchShape{};
     }
     s.G = G;
     s.acc = acc;
@@ -470,7 +422,8 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     s.spad = scap + ((want - scap) % mod + mod) % mod;
     s.TS = ts;
     s.threads = G * ts;
-    s.smem = (size_t)ts * s.spad * esize(a) + 5 * sizeof(uint32_t) * ts + (s.fx ? ts * sizeof(FxGeo) : 0);
+    s.smem = (size_t)ts * s.spad * esize(a) + 5 * sizeof(uint32_t) * ts +
+             (s.fx && a != Arith::FFQ && a != Arith::FF ? ts * sizeof(FxGeo) : 0);
     if (s.smem > 232448) return LaunchShape{};
     return s;
 }
@@ -521,7 +474,7 @@ LaunchShape best_shape(Arith a, int P, int G, bool small_tiles, int min_threads)
                 best[k] = s;
             }
         }
-    if (!best[0].acc || (best[0].fx && 8 * most[1] >= 9 * most[0])) return best[1];
+    if (!best[0].acc || (a == Arith::F64 && 8 * most[1] >= 9 * most[0])) return best[1];
     return best[0];
 }
 
@@ -615,12 +568,13 @@ void sfmm_destroy(sfmm_context *c)
 {
     if (!c) return;
     cudaSetDevice(c->device);
-    for (auto &t : c->tab) free_tables(t);
+    free_tables(c->tab);
     for (auto &t : c->tc) tc_release(t);
-    for (auto &t : c->fxt) free_fx(t);
-    for (auto &t : c->f32t) free_fx(t);
-    for (void *p : c->fx_edge)
-        if (p) cudaFree(p);
+    for (auto &ts : c->fxt)
+        for (auto &t : ts) free_fx(t);
+    for (auto &es : c->fx_edge)
+        for (void *p : es)
+            if (p) cudaFree(p);
     for (int k = 0; k < 3; ++k) {
         c->d_src[k].release();
         c->d_dst[k].release();

@@ -23,16 +23,15 @@
 
 namespace sfmm {
 
+// device tables of the FP64 kernel for orders above 32
 struct DevTables {
     void *W = nullptr, *ein_M = nullptr, *ein_L = nullptr, *eout_L = nullptr, *eout_M = nullptr;
     void *H[3] = {nullptr, nullptr, nullptr};
-    void *Wq = nullptr;  // Q1.30 swap matrices (fixed-point variant only)
-    void *W8 = nullptr, *Wq8 = nullptr;  // 8-row padded copies (HostTables::W8), contexts above order 32
     bool ready = false;
 };
 
-// device tables of the 60-bit fixed-point or the FP32 kernel (sfmm_tables.hpp,
-// FxTables and F32Tables), one set per group size; the edge factors (e_in_M,
+// device tables of the 60-bit fixed-point, the FP32 or the split kernel
+// (sfmm_tables.hpp, FxTables, F32Tables, SplitTables), one set per group size; the edge factors (e_in_M,
 // e_in_L, e_out_L, e_out_M) are shared by the sets
 struct FxDevTables {
     void *W = nullptr, *H[3] = {nullptr, nullptr, nullptr};
@@ -94,9 +93,9 @@ struct sfmm_context {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     sfmm::HostTables host;
-    sfmm::DevTables tab[sfmm::kNumArith];  // indexed by Arith (the tensor-core modes use tc[])
-    sfmm::FxDevTables fxt[2], f32t[2];  // 4 and 8 threads per translation
-    void *fx_edge[4] = {nullptr, nullptr, nullptr, nullptr};
+    sfmm::DevTables tab;  // FP64 above order 32
+    sfmm::FxDevTables fxt[sfmm::kNumArith][2];  // by Arith, 4 and 8 threads per translation
+    void *fx_edge[sfmm::kNumArith][4] = {};
     sfmm::TcDevTables *tc[3] = {nullptr, nullptr, nullptr};  // tensor-core operand images by format
     std::string err;
     std::atomic<uint64_t> launches{0};
@@ -112,8 +111,7 @@ struct sfmm_context {
     // (op, arith, order bound) -> launch shape: operators tuned apart keep
     // their own shapes at one order
     std::map<std::tuple<int, int, int>, sfmm::LaunchShape> shapes;
-    int *d_woff = nullptr, *d_hoff = nullptr;            // table offsets (shared by all arithmetics)
-    int *d_woff8 = nullptr;                              // offsets of the 8-row padded swap blocks
+    int *d_woff = nullptr, *d_hoff = nullptr;            // offsets of tab's blocks
     bool pageable_access = false;  // the GPU reads pageable host memory through the host page tables
     sfmm::SlotScratch slot_scratch;  // target table of the classic host call
     std::set<std::tuple<int, int, int>> tuned;  // (op, arith, order bound) shapes measured by sfmm_tune

@@ -21,6 +21,14 @@
 
 namespace sfmm {
 
+// a b with subnormal operands and results flushed to zero
+__device__ __forceinline__ float mul_ftz(float a, float b)
+{
+    float r;
+    asm("mul.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // fixed-point Q60 value (limbs) to FP32
 __device__ __forceinline__ float f32_of_fx(fx v)
 {

@@ -79,64 +79,11 @@ __device__ __forceinline__ int group_renorm_shift(const long long (&ar)[NA], con
     return used > kFixBits ? used - kFixBits : 0;
 }
 
-__device__ __forceinline__ int round_shift(long long a, int s)
-{
-    return s ? (int)((a + (1ll << (s - 1))) >> s) : (int)a;
-}
-
 // (c*x - s*y) in Q1.30, rounded
 __device__ __forceinline__ int rot_q30(int c, int x, int s, int y)
 {
     const long long t = (long long)c * x - (long long)s * y;
     return (int)((t + (1ll << 29)) >> 30);
-}
-
-// Integer swap of one degree, both parts: rows i = q + G a (a < NA) of the
-// Q1.30 matrices applied to the int32 mantissas stored in the buffer slots
-// (low word of each 8-byte slot).  Same coefficient layout (slot t: R rows of
-// W_R, then R rows of W_I), padding and software pipelining as the
-// floating-point swap.
-template <int G, int NA, int R>
-__device__ __forceinline__ void swap_both_fixed(const int *__restrict__ W, const float2 *xre, const float2 *xim,
-                                                int d, int n, int q, long long (&ar)[NA], long long (&ai)[NA])
-{
-    const int jr0 = (q + n) & 1, ji0 = jr0 ^ 1;
-    const int cnt = (d + 1) >> 1;
-    const int *w = W + q;
-    const int *xr_p = reinterpret_cast<const int *>(xre + jr0);
-    const int *xi_p = reinterpret_cast<const int *>(xim + ji0);
-    int xrn = *xr_p, xin = *xi_p;
-    int wrn[NA], win[NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        wrn[a] = __ldg(w + G * a);
-        win[a] = __ldg(w + R + G * a);
-    }
-#pragma unroll 4  // measured on GB300: 4 beats 2 by 0.6% at P=16, 8 and 1 lose
-    for (int t = 0; t < cnt; ++t) {
-        const int xr = xrn, xi = xin;
-        int wr[NA], wi[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            wr[a] = wrn[a];
-            wi[a] = win[a];
-        }
-        xr_p += 4;  // two 8-byte slots
-        xi_p += 4;
-        w += 2 * R;
-        xrn = *xr_p;
-        xin = *xi_p;
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            wrn[a] = __ldg(w + G * a);
-            win[a] = __ldg(w + R + G * a);
-        }
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            ar[a] += (long long)wr[a] * xr;
-            ai[a] += (long long)wi[a] * xi;
-        }
-    }
 }
 
 }  // namespace sfmm

@@ -1,10 +1,8 @@
-// Fused translation kernels, double arithmetic.
+// FP64 translations above order 32, one warp per translation.
 #include "sfmm_kernel_impl.cuh"
 
 namespace sfmm {
-cudaError_t launch_translate_64(const KParams &p, const LaunchShape &s, int grid, cudaStream_t st)
-{
-    return launch_typed<double>(p, s, grid, st);
-}
-int occupancy_64(const LaunchShape &s) { return occupancy_typed<double>(s); }
+#define SHAPES(X, K) X(K, 32, 2) X(K, 32, 3)
+#define KERNEL(G, ACC, HBM, WORK) (k_translate<double, G, ACC, false, HBM, WORK>)
+SFMM_DEFINE_LAUNCH(launch_translate_64, occupancy_64, SHAPES, KERNEL)
 }  // namespace sfmm

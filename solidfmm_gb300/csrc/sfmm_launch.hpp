@@ -39,7 +39,7 @@ struct LaunchShape {
     int spad = 0;      // buffer elements per translation
     size_t smem = 0;   // dynamic shared memory bytes
     int threads = 0;   // G * TS
-    bool fx = false;   // the 60-bit fixed-point kernel (FP64)
+    bool fx = false;   // tables by group size (every kernel but FP64 above order 32)
     int blocks_per_sm = 0;  // resident CTAs per SM (occupancy of this shape)
 };
 

@@ -46,7 +46,6 @@ struct KParams {
     int atomic;
     int in_hbm;    // expansions in device memory (0: host memory read over the link)
     const void *W;      // arith-typed swap matrices (padded, see sfmm_tables.hpp)
-    const int *Wq;      // swap matrices in Q1.30 (fixed-point variant), same layout as W
     const int *woff;    // offset of degree n's W blocks
     const int *hoff;    // offset of column m's z matrix
     int rowpad;         // row padding of W and H blocks (8 or 32)

@@ -259,6 +259,51 @@ F32Tables build_f32_tables(const HostTables &t, int G, int P)
     return f;
 }
 
+SplitTables build_split_tables(const HostTables &t, int G, int P)
+{
+    SplitTables f;
+    f.woff.resize(P);
+    size_t tot = 0;
+    for (int n = 0; n < P; ++n) {
+        f.woff[n] = (int)tot;
+        tot += size_t((n + 2) / 2) * ((n + G) / G) * G;
+    }
+    f.W.assign(2 * (tot + size_t((P + G - 1) / G) * G), 0);  // and a slot that the last degree's loop loads ahead
+    for (int n = 0; n < P; ++n) {
+        const int d = n + 1, NA = (d + G - 1) / G;
+        for (int tt = 0; tt < (d + 1) / 2; ++tt)
+            for (int q = 0; q < G; ++q)
+                for (int a = 0; a < NA; ++a) {
+                    const int jr = (q + n) & 1, i = q + G * a;
+                    const size_t in_slot = a / 2 * 2 + 1 < NA ? size_t(a / 2 * G + q) * 2 + (a & 1) : size_t(NA - 1) * G + q;
+                    int32_t *at = &f.W[2 * (f.woff[n] + size_t(tt) * NA * G + in_slot)];
+                    at[0] = (int32_t)std::llround(std::ldexp(w_entry(t, n, 0, i, jr + 2 * tt), 30));
+                    at[1] = (int32_t)std::llround(std::ldexp(w_entry(t, n, 1, i, (jr ^ 1) + 2 * tt), 30));
+                }
+    }
+    f.hoff.resize(P);
+    tot = 0;
+    for (int m = 0; m < P; ++m) {
+        f.hoff[m] = (int)tot;
+        tot += size_t(P - m) * fx_hrow(P - m, 2 * G);
+    }
+    for (int op = 0; op < 3; ++op) {
+        f.H[op].assign(2 * tot, 0.f);
+        for (int m = 0; m < P; ++m) {
+            const int HR = hrows(t.P - m, t.pad), hs = fx_hrow(P - m, 2 * G);
+            for (int k = 0; k < P - m; ++k)
+                for (int np = 0; np < P - m; ++np) {
+                    const int q = np % G, b = np / G;
+                    const double v = t.H[op][t.hoff[m] + size_t(k) * HR + np];
+                    float *at = &f.H[op][2 * (f.hoff[m] + size_t(k) * hs + b / 2 * 2 * G + 2 * q + (b & 1))];
+                    at[0] = (float)v;
+                    at[1] = (float)(v - (double)at[0]);
+                }
+        }
+    }
+    return f;
+}
+
 std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count)
 {
     std::vector<int32_t> out(4 * count);

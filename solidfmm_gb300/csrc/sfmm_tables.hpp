@@ -102,6 +102,18 @@ struct F32Tables {
     std::vector<int> woff, hoff;
 };
 F32Tables build_f32_tables(const HostTables &t, int G, int P);
+// Tables of the split kernel: swap coefficients round(w 2^30) as (W_R, W_I)
+// pairs, degree n at woff[n] (in pairs, one more slot after the last), slot t (column jr + 2t of W_R, (jr ^
+// 1) + 2t of W_I, jr = (q + n) & 1) NA G further, rows i = q + G a of lane q:
+// for each pair a = 2p, 2p + 1 at (p G + q) 2, an odd last row at (NA - 1) G + q.
+// z matrices as float-float pairs (hi, lo), output n' = m + q + G b at (b / 2)
+// 2 G + 2 q + (b & 1) of a row of fx_hrow(P - m, 2 G) entries.
+struct SplitTables {
+    std::vector<int32_t> W;
+    std::vector<float> H[3];
+    std::vector<int> woff, hoff;
+};
+SplitTables build_split_tables(const HostTables &t, int G, int P);
 // positive edge factors as (h, l, exponent, 0): (h 2^30 + l) 2^(exponent - 60)
 std::vector<int32_t> fx_edges(const std::vector<double> &e, size_t count);
 

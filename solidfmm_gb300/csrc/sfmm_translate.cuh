@@ -17,13 +17,13 @@
 //      microkernel_generic.cpp:362-380), with FP64/FP32 atomics when
 //      targets may repeat.
 //
-// Thread q of a group owns rows i = q + G a of every degree-n swap,
-// rotation elements m = q + G a, and outputs n' = m + q + G a of every
-// z-translation column; each stage keeps its accumulators in registers and
-// reads its inputs from the buffer (group members synchronise with
-// __syncwarp).  The number of accumulator blocks a stage needs,
-// ceil(d / G), is warp-uniform and selects a stage instance compiled for
-// exactly that many blocks, so no block is issued only to be predicated off.
+// Thread q of a group owns every G-th (or, holding one part of an element,
+// every (G/2)-th) row of a degree and output of a z-translation column; each
+// stage keeps its accumulators in registers and reads its inputs from the
+// buffer (group members synchronise with __syncwarp).  The number of
+// accumulator blocks a stage needs is warp-uniform and selects a stage instance
+// compiled for exactly that many blocks, so no block is issued only to be
+// predicated off.
 // Loop bounds are warp-uniform maxima over the warp's 32/G translations,
 // like the reference's lanes padded with zero orders (translations.cpp:504-514);
 // inputs past a translation's own order read as zero and outputs past it are
@@ -34,9 +34,9 @@
 #include <type_traits>
 
 #include "sfmm_arith.cuh"
-#include "sfmm_fixed.cuh"
 #include "sfmm_f32.cuh"
 #include "sfmm_fx.cuh"
+#include "sfmm_split.cuh"
 #include "sfmm_params.hpp"
 
 namespace sfmm {
@@ -108,21 +108,18 @@ __device__ __forceinline__ void for_columns(int m, int mend, int nout, F &&f)
         if (m < mend) for_columns<NB - 1, RS>(m, mend, nout, f);
 }
 
-// Rows of a degree's swap-coefficient block in the instance that runs NA
-// accumulator blocks of G threads: the tables pad rows to a multiple of 8
-// for orders up to 32 (G = 4 or 8) and of 32 above (G = 32), so the row
-// count of every degree served by one (G, NA) instance is the same
-// compile-time constant.
-// The two swap passes of a degree: unrolled for FP64 and FP32 (the second
-// pass's loads overlap the first's tail: +1.8% FP64, +3% FP32 at P=20 on
-// GB300), rolled for float-float (-5% unrolled)
-template <class T>
-constexpr int kPassUnroll = std::is_same<T, double>::value || std::is_same<T, float>::value ? 2 : 1;
+// The stages below, down to the geometry, are those of the FP64 kernel for
+// orders above 32 (one warp per translation, both parts of an element in one
+// lane); the other kernels' are in sfmm_fx.cuh, sfmm_f32.cuh and sfmm_split.cuh.
 
+// Rows of a degree's swap-coefficient block in the instance that runs NA
+// accumulator blocks: the tables pad rows to a multiple of 32 above order 32,
+// so the row count of every degree served by one instance is the same
+// compile-time constant.
 template <int G, int NA>
 __host__ __device__ constexpr int swap_rows()
 {
-    return G == 32 ? 32 * NA : ((G * NA + 7) & ~7);
+    return G * NA;
 }
 
 // Both swap parts of one degree: rows i = q + G a (a < NA) of W_R applied to
@@ -143,10 +140,6 @@ __device__ __forceinline__ void swap_both(const typename AR::T *__restrict__ W, 
 {
     using T = typename AR::T;
     constexpr int R = swap_rows<G, NA>();
-    // unrolling measured on GB300: FP64 runs best rolled (its pipe is the
-    // limit; +3% at M2L P=16), FP32 unrolled four times (+7% at P=16 with the
-    // passes unrolled too), float-float twice (-10% rolled)
-    constexpr int kUnroll = std::is_same<T, double>::value ? 1 : (std::is_same<T, float>::value ? 4 : 2);
     const int jr0 = (q + n) & 1, ji0 = jr0 ^ 1;
     const int cnt = (d + 1) >> 1;  // iterations of the longer part
     const T *w = W + q;
@@ -159,7 +152,7 @@ __device__ __forceinline__ void swap_both(const typename AR::T *__restrict__ W, 
         wrn[a] = AR::ldt(w + G * a);
         win[a] = AR::ldt(w + R + G * a);
     }
-#pragma unroll kUnroll
+#pragma unroll 1  // the FP64 pipe is the limit
     for (int t = 0; t < cnt; ++t) {
         const T xr = xrn, xi = xin;
         T wr[NA], wi[NA];
@@ -219,7 +212,7 @@ __device__ __forceinline__ void forward_degree(typename AR::Stor *b, int n,
         }
     }
     __syncwarp();
-#pragma unroll kPassUnroll<typename AR::T>
+#pragma unroll 2
     for (int pass = 0; pass < 2; ++pass) {
         Acc ar[NA], ai[NA];
 #pragma unroll
@@ -262,7 +255,7 @@ __device__ __forceinline__ void backward_degree(typename AR::Stor *b, int n,
     const int d = n + 1;
     S *bre = b + n * (n + 1);
     S *bim = b + (n + 1) * (n + 1);
-#pragma unroll kPassUnroll<typename AR::T>
+#pragma unroll 2
     for (int pass = 0; pass < 2; ++pass) {
         Acc ar[NA], ai[NA];
 #pragma unroll
@@ -293,143 +286,6 @@ __device__ __forceinline__ void backward_degree(typename AR::Stor *b, int n,
                 }
                 AR::st(bre + ii, vr);
                 AR::st(bim + ii, vi);
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// Q1.30 cos / sin of m beta for the rotation elements a thread owns
-template <int ACC>
-struct FixTrig {
-    int c[ACC], s[ACC];
-};
-
-__device__ __forceinline__ void st_fixed(float2 *p, int v) { *reinterpret_cast<int *>(p) = v; }
-
-// One degree of the forward transform with the swaps and the beta rotation
-// in block fixed point: float-float edge, conversion at the row's block
-// exponent, integer swap, renormalise, integer rotation, integer swap,
-// renormalise, back to float-float.
-template <int G, int NA, int ACC>
-__device__ __forceinline__ void forward_degree_fixed(float2 *b, int n, const int *__restrict__ WRq,
-                                                     const ff *__restrict__ ein, ff f, int q,
-                                                     const Trig<arith<ff>, ACC> &tg, const FixTrig<ACC> &tq)
-{
-    using AR = arith<ff>;
-    const int d = n + 1;
-    float2 *bre = b + n * (n + 1);
-    float2 *bim = b + (n + 1) * (n + 1);
-    ff vr[NA], vi[NA];
-    float mx = 0.f;
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = q + G * a;
-        vr[a] = vi[a] = AR::zero();
-        if (m < d) {
-            const ff xr = AR::ld(bre + m);
-            const ff xi = AR::ld(bim + m);
-            const ff g = AR::mul(f, AR::ldt(ein + m));
-            const ff gc = AR::mul(g, tg.ca[a]), gs = AR::mul(g, tg.sa[a]);
-            vr[a] = AR::dot2(gc, xr, AR::neg(gs), xi);
-            vi[a] = AR::dot2(gs, xr, gc, xi);
-            mx = fmaxf(mx, fmaxf(fabsf(vr[a].hi), fabsf(vi[a].hi)));
-        }
-    }
-    int E = block_exponent(group_max<G>(mx));
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = q + G * a;
-        if (m < d) {
-            st_fixed(bre + m, ff_to_fixed(vr[a], E));
-            st_fixed(bim + m, ff_to_fixed(vi[a], E));
-        }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-        long long ar[NA], ai[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) ar[a] = ai[a] = 0;
-        swap_both_fixed<G, NA, swap_rows<G, NA>()>(WRq, bre, bim, d, n, q, ar, ai);
-        const int sh = group_renorm_shift<G, NA>(ar, ai);
-        E += sh - 30;
-        __syncwarp();
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            const int ii = q + G * a;
-            if (ii < d) {
-                const int xr = round_shift(ar[a], sh), xi = round_shift(ai[a], sh);
-                if (pass == 0) {  // rotation by e^{+i m beta} between the two swaps
-                    st_fixed(bre + ii, rot_q30(tq.c[a], xr, tq.s[a], xi));
-                    st_fixed(bim + ii, rot_q30(tq.c[a], xi, -tq.s[a], xr));
-                } else {
-                    AR::st(bre + ii, fixed_to_ff(xr, E));
-                    AR::st(bim + ii, fixed_to_ff(xi, E));
-                }
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// One degree of the backward transform with fixed-point swaps and beta
-// rotation; the alpha rotation and r-power scale stay in float-float.
-template <int G, int NA, int ACC>
-__device__ __forceinline__ void backward_degree_fixed(float2 *b, int n, const int *__restrict__ WRq,
-                                                      const ff *__restrict__ eout, ff f, int q,
-                                                      const Trig<arith<ff>, ACC> &tg, const FixTrig<ACC> &tq)
-{
-    using AR = arith<ff>;
-    const int d = n + 1;
-    float2 *bre = b + n * (n + 1);
-    float2 *bim = b + (n + 1) * (n + 1);
-    ff vr[NA], vi[NA];
-    float mx = 0.f;
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = q + G * a;
-        vr[a] = vi[a] = AR::zero();
-        if (m < d) {
-            vr[a] = AR::ld(bre + m);
-            vi[a] = AR::ld(bim + m);
-            mx = fmaxf(mx, fmaxf(fabsf(vr[a].hi), fabsf(vi[a].hi)));
-        }
-    }
-    int E = block_exponent(group_max<G>(mx));
-#pragma unroll
-    for (int a = 0; a < NA; ++a) {
-        const int m = q + G * a;
-        if (m < d) {
-            st_fixed(bre + m, ff_to_fixed(vr[a], E));
-            st_fixed(bim + m, ff_to_fixed(vi[a], E));
-        }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {
-        long long ar[NA], ai[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) ar[a] = ai[a] = 0;
-        swap_both_fixed<G, NA, swap_rows<G, NA>()>(WRq, bre, bim, d, n, q, ar, ai);
-        const int sh = group_renorm_shift<G, NA>(ar, ai);
-        E += sh - 30;
-        __syncwarp();
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            const int ii = q + G * a;
-            if (ii < d) {
-                const int xr = round_shift(ar[a], sh), xi = round_shift(ai[a], sh);
-                if (pass == 0) {  // e^{-i m beta}
-                    st_fixed(bre + ii, rot_q30(tq.c[a], xr, -tq.s[a], xi));
-                    st_fixed(bim + ii, rot_q30(tq.c[a], xi, tq.s[a], xr));
-                } else {  // e^{-i m alpha}, back to the solid basis, r-power scale
-                    const ff ur = fixed_to_ff(xr, E), ui = fixed_to_ff(xi, E);
-                    const ff g = AR::mul(f, AR::ldt(eout + ii));
-                    const ff gc = AR::mul(g, tg.ca[a]), gs = AR::mul(g, tg.sa[a]);
-                    AR::st(bre + ii, AR::dot2(gc, ur, gs, ui));
-                    AR::st(bim + ii, AR::dot2(gc, ui, AR::neg(gs), ur));
-                }
             }
         }
         __syncwarp();
@@ -557,63 +413,62 @@ __device__ __forceinline__ float src_scaled(float x, int e, const float *) { ret
 // beyond the FP32 range come into it
 __device__ __forceinline__ float src_scaled(double x, int e, const float *) { return (float)d_scaled(x, e); }
 
-// Per-thread geometry of one translation: |shift|, its inverse and the
-// rotation factors.  FP64 for the FP64 and FP32 kernels; float-float for the
-// split kernels, which then execute no FP64 instruction here (GB300's FP64
-// pipe runs at 1/64 of the FP32 rate).
-template <class AR, int G, int ACC, bool FIX>
+// Per-thread geometry of one translation in FP64 (orders above 32): |shift|,
+// its inverse and the rotation factors.
+template <class AR, int G, int ACC>
 struct Geometry {
-    using T = typename AR::T;
-    T r, rinv;           // |shift| and 1/|shift| in the arithmetic
-    double rd, rinvd;    // the same in FP64 (FP64 and FP32 kernels)
+    double r, rinv;
     Trig<AR, ACC> tg;
-    FixTrig<ACC> tq;
 
     __device__ __forceinline__ Geometry(double x, double y, double z, int q)
     {
-        if constexpr (AR::split) {
-            using A = arith<ff>;
-            const ff fx = ff_from_d_int(x), fy = ff_from_d_int(y), fz = ff_from_d_int(z);
-            const ff rxy2 = A::dot2(fx, fx, fy, fy);
-            const ff rxy = ff_sqrt(rxy2);
-            r = ff_sqrt(A::add(rxy2, A::mul(fz, fz)));
-            rinv = ff_rcp(r);
-            rd = rinvd = 0.0;
-            cff ea{ff{1.f, 0.f}, ff{0.f, 0.f}};
-            if (rxy.hi > 0.f) {
-                const ff rr = ff_rcp(rxy);
-                ea = cff{A::mul(fy, rr), A::mul(fx, rr)};
-            }
-            const cff eb{A::mul(fz, rinv), A::neg(A::mul(rxy, rinv))};
-            auto cm = [](cff a, cff b) {
-                return cff{A::dot2(a.c, b.c, A::neg(a.s), b.s), A::dot2(a.s, b.c, a.c, b.s)};
-            };
-            rotation_powers<G, ACC>(ea, eb, cff{ff{1.f, 0.f}, ff{0.f, 0.f}}, q, cm, [&](int a, cff pa, cff pb) {
-                tg.ca[a] = pa.c;
-                tg.sa[a] = pa.s;
-                tg.cb[a] = pb.c;
-                tg.sb[a] = pb.s;
-                if constexpr (FIX) {  // Q1.30
-                    tq.c[a] = __float2int_rn(pb.c.hi * 1073741824.f) + __float2int_rn(pb.c.lo * 1073741824.f);
-                    tq.s[a] = __float2int_rn(pb.s.hi * 1073741824.f) + __float2int_rn(pb.s.lo * 1073741824.f);
-                }
-            });
-        } else {
-            const double rxy = hypot(x, y);
-            rd = hypot(rxy, z);
-            rinvd = 1.0 / rd;
-            r = AR::from_d(rd);
-            rinv = AR::from_d(rinvd);
-            const cd ea = (rxy == 0) ? cd{1.0, 0.0} : cd{y / rxy, x / rxy};
-            const cd eb = cd{z * rinvd, -rxy * rinvd};
-            rotation_powers<G, ACC>(ea, eb, cd{1.0, 0.0}, q, [](cd a, cd b) { return cmul(a, b); },
-                                    [&](int a, cd pa, cd pb) {
-                                        tg.ca[a] = AR::from_d(pa.c);
-                                        tg.sa[a] = AR::from_d(pa.s);
-                                        tg.cb[a] = AR::from_d(pb.c);
-                                        tg.sb[a] = AR::from_d(pb.s);
-                                    });
+        const double rxy = hypot(x, y);
+        r = hypot(rxy, z);
+        rinv = 1.0 / r;
+        const cd ea = (rxy == 0) ? cd{1.0, 0.0} : cd{y / rxy, x / rxy};
+        const cd eb = cd{z * rinv, -rxy * rinv};
+        rotation_powers<G, ACC>(ea, eb, cd{1.0, 0.0}, q, [](cd a, cd b) { return cmul(a, b); },
+                                [&](int a, cd pa, cd pb) {
+                                    tg.ca[a] = pa.c;
+                                    tg.sa[a] = pa.s;
+                                    tg.cb[a] = pb.c;
+                                    tg.sb[a] = pb.s;
+                                });
+    }
+};
+
+// The same in float-float for the split kernel, which executes no FP64
+// instruction here (GB300's FP64 pipe runs at 1/64 of the FP32 rate).
+template <int G, int ACC>
+struct SplitGeometry {
+    ff r, rinv;
+    FFTrig<ACC> tg;
+    FixTrig<ACC> tq;
+
+    __device__ __forceinline__ SplitGeometry(double x, double y, double z, int q)
+    {
+        using A = arith<ff>;
+        const ff fx = ff_from_d_int(x), fy = ff_from_d_int(y), fz = ff_from_d_int(z);
+        const ff rxy2 = A::dot2(fx, fx, fy, fy);
+        const ff rxy = ff_sqrt(rxy2);
+        r = ff_sqrt(A::add(rxy2, A::mul(fz, fz)));
+        rinv = ff_rcp(r);
+        cff ea{ff{1.f, 0.f}, ff{0.f, 0.f}};
+        if (rxy.hi > 0.f) {
+            const ff rr = ff_rcp(rxy);
+            ea = cff{A::mul(fy, rr), A::mul(fx, rr)};
         }
+        const cff eb{A::mul(fz, rinv), A::neg(A::mul(rxy, rinv))};
+        auto cm = [](cff a, cff b) {
+            return cff{A::dot2(a.c, b.c, A::neg(a.s), b.s), A::dot2(a.s, b.c, a.c, b.s)};
+        };
+        rotation_powers<G, ACC>(ea, eb, cff{ff{1.f, 0.f}, ff{0.f, 0.f}}, q, cm, [&](int a, cff pa, cff pb) {
+            tg.ca[a] = pa.c;
+            tg.sa[a] = pa.s;
+            // Q1.30
+            tq.c[a] = __float2int_rn(pb.c.hi * 1073741824.f) + __float2int_rn(pb.c.lo * 1073741824.f);
+            tq.s[a] = __float2int_rn(pb.s.hi * 1073741824.f) + __float2int_rn(pb.s.lo * 1073741824.f);
+        });
     }
 };
 
@@ -637,11 +492,8 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     constexpr bool PL = FIX && !AR::split;
     constexpr bool F32 = std::is_same<A, float>::value;
 
-    // Loads in flight per lane in the source gather and the target update,
-    // measured on GB300 (M2L P=16, 10^6): 8 and 4 make the split kernel 2.2%
-    // and the FP32 kernel 3.7% faster than 4 and 1, which the FP64 and
-    // float-float kernels keep (1.5% and 0.7% slower with 8 and 4).
-    constexpr bool kDeep = FIX;
+    // loads in flight per lane in the source gather and the target update
+    // (M2L P=16 x 10^6, split: 8 and 4 over 4 and 1 are worth 2.2%)
     // FP32-range arithmetics run every translation at the length scale of
     // its shift: lambda = 2^ks with |shift| / lambda in [2, 7), sources (and
     // the shift) divided by lambda^n (multipoles) or lambda^-(n+1) (locals),
@@ -652,8 +504,7 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     // inside the FP32 range at every geometry scale; shifts whose largest
     // component lies in [2, 4) run unscaled
     constexpr bool kScale = !std::is_same<A, double>::value;
-    constexpr int kGatherUnroll = kDeep ? 8 : 4;
-    constexpr int kAccUnroll = kDeep ? 4 : 1;
+    constexpr int kGatherUnroll = FIX ? 8 : 4;
     constexpr int kAccBatch = 5;
 
     extern __shared__ __align__(16) unsigned char smem[];
@@ -683,13 +534,14 @@ __device__ __forceinline__ void translate_body(const KParams &p)
     const Src *src = reinterpret_cast<const Src *>(p.src);
     Src *dst = reinterpret_cast<Src *>(p.dst);
     const int op = p.op;
-    if constexpr (PL) {
+    if constexpr (FIX) {
         // this order's tables into L1, all loads in flight at once (the
         // transforms would meet them one miss after the other)
         touch_tables(p.W, p.wbytes);
         touch_tables(p.H, p.hbytes);
-        touch_tables(p.ein, P * (P + 1) / 2 * (F32 ? 4 : 16));
-        touch_tables(p.eout, P * (P + 1) / 2 * (F32 ? 4 : 16));
+        constexpr int kEdge = F32 ? 4 : AR::split ? 8 : 16;
+        touch_tables(p.ein, P * (P + 1) / 2 * kEdge);
+        touch_tables(p.eout, P * (P + 1) / 2 * kEdge);
     }
 
     for (long long tile = blockIdx.x;; tile += gridDim.x) {
@@ -797,12 +649,12 @@ __device__ __forceinline__ void translate_body(const KParams &p)
                 const int es = op == OP_L2L ? ksg : -ksg;  // per degree
                 const int e0 = op == OP_L2L ? ksg : 0;
                 if constexpr (F32) {
-                    // every factor an FP32 normal: plain products (a result
-                    // below the normal range keeps what digits it has)
+                    // every factor an FP32 normal: a product does it, with
+                    // subnormals flushed as f_scaled does
                     if (abs(es) * P + abs(e0) <= 126) {
 #pragma unroll(kGatherUnroll)
                         for (int c = lane; c < p.spad; c += 32)
-                            bp[c] = c < cnt ? __ldcs(sp + c) * pow2f(es * degree_at(c) + e0) : 0.f;
+                            bp[c] = c < cnt ? mul_ftz(__ldcs(sp + c), pow2f(es * degree_at(c) + e0)) : 0.f;
                         continue;
                     }
                 }
@@ -947,79 +799,80 @@ __device__ __forceinline__ void translate_body(const KParams &p)
                 e += n + 1;
                 f = fxs_mul(f, bstep);
             });
+        } else if constexpr (AR::split) {
+            const SplitGeometry<G, ACC> geo(x, y, z, q);
+            // 2. forward transforms: r^n (L input) or r^-(n+1) (M input), by
+            // repeated multiplication (error ~n 2^-48)
+            const ff one{1.f, 0.f};
+            ff f = op == OP_L2L ? one : geo.rinv;
+            const ff fstep = op == OP_L2L ? geo.r : geo.rinv;
+            const int2 *w = reinterpret_cast<const int2 *>(p.W);
+            const T *e = EIN;
+            for_degrees<ACC, G>(pin_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                forward_degree_split<G, NA, ACC>(b, n, w, e, f, q, geo.tg, geo.tq);
+                w += ((n + 2) >> 1) * (NA * G);
+                e += n + 1;
+                f = ff_mul(f, fstep);
+            });
+            // 3. z-translation (columns m >= min(P_in, P_out) of the outputs
+            // stay zero: their rows beyond P_in were zero-filled by the gather)
+            const float2 *h = reinterpret_cast<const float2 *>(p.H);
+            for_columns<ACC, G>(0, min(pin_w, pout_w), pout_w, [&](auto nb, int m) {
+                const int hs = fx_hrow(p.Ptab - m, 2 * G);
+                z_column_split<G, decltype(nb)::value>(b, h, hs, m, op == OP_L2L ? m + q : m,
+                                                       op == OP_M2M ? min(pin_w, pout_w) : pin_w, pout_w, q);
+                h += (p.Ptab - m) * hs;
+            });
+            // 4. backward transforms: r^(n+1) (M output) or r^-n (L output)
+            f = op == OP_M2M ? geo.r : one;
+            const ff bstep = op == OP_M2M ? geo.r : geo.rinv;
+            w = reinterpret_cast<const int2 *>(p.W);
+            e = EOUT;
+            for_degrees<ACC, G>(pout_w, [&](auto na, int n) {
+                constexpr int NA = decltype(na)::value;
+                backward_degree_split<G, NA, ACC>(b, n, w, e, f, q, geo.tg, geo.tq);
+                w += ((n + 2) >> 1) * (NA * G);
+                e += n + 1;
+                f = ff_mul(f, bstep);
+            });
         } else {
             // geometry (euler, microkernel_generic.cpp:37-97)
-            Geometry<AR, G, ACC, FIX> geo(x, y, z, q);
-            const Trig<AR, ACC> &tg = geo.tg;
-            const FixTrig<ACC> &tq = geo.tq;
-
-            // 2. forward transforms, degree by degree
-            const bool Lin = (op == OP_L2L);
-            // r-power scale of degree n: r^n (L input) or r^-(n+1) (M input).
-            // Float-float steps by repeated multiplication (FP32 pipe, error
-            // ~n 2^-48); FP64 and FP32 take every power from the FP64 product.
-            constexpr bool kFF = AR::split;
-            double rp = Lin ? 1.0 : geo.rinvd;
-            const double rpstep = Lin ? geo.rd : geo.rinvd;
-            T f = Lin ? AR::from_d(1.0) : geo.rinv;
-            const T rstep = Lin ? geo.r : geo.rinv;
+            const Geometry<AR, G, ACC> geo(x, y, z, q);
+            // 2. forward transforms, degree by degree; r-power scale of degree
+            // n: r^n (L input) or r^-(n+1) (M input)
+            T f = op == OP_L2L ? 1.0 : geo.rinv;
+            const T fstep = op == OP_L2L ? geo.r : geo.rinv;
             for (int n = 0; n < pin_w; ++n) {
-                if (!kFF) f = AR::from_d(rp);
-                const T *ein = EIN + n * (n + 1) / 2;
-                if constexpr (FIX) {
-                    const int *WRq = p.Wq + __ldg(p.woff + n);
-                    dispatch<ACC>((n + G) / G, [&](auto na) {
-                        forward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, ein, f, q, tg, tq);
-                    });
-                } else {
-                    const T *WR = W + __ldg(p.woff + n);
-                    dispatch<ACC>((n + G) / G, [&](auto na) {
-                        forward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, ein, f, q, tg);
-                    });
-                }
-                if (kFF) f = AR::mul(f, rstep);
-                if (!kFF) rp *= rpstep;
+                const T *WR = W + __ldg(p.woff + n);
+                dispatch<ACC>((n + G) / G, [&](auto na) {
+                    forward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, EIN + n * (n + 1) / 2, f, q, geo.tg);
+                });
+                f *= fstep;
             }
-
             // 3. z-translation, column by column.  Columns m >= min(P_in, P_out)
             //    of the outputs stay zero (trans2swap_buf, microkernel_generic.cpp:308-338):
             //    their rows beyond P_in were zero-filled by the gather.
-            const int nout_w = pout_w;
             const int mend = min(pin_w, pout_w);
             for (int m = 0; m < mend; ++m) {
                 const int HR = (p.Ptab - m + p.rowpad - 1) & ~(p.rowpad - 1);
                 const T *Hm = H + __ldg(p.hoff + m);
                 // M2M only needs inputs k <= n' and L2L only k >= n'
                 const int kbeg = (op == OP_L2L) ? m + q : m;
-                const int kend = (op == OP_M2M) ? min(pin_w, nout_w) : pin_w;
-                dispatch<ACC>((nout_w - m + G - 1) / G, [&](auto na) {
-                    z_column<AR, G, decltype(na)::value>(b, Hm, HR, m, kbeg, kend, nout_w, q);
+                const int kend = (op == OP_M2M) ? mend : pin_w;
+                dispatch<ACC>((pout_w - m + G - 1) / G, [&](auto na) {
+                    z_column<AR, G, decltype(na)::value>(b, Hm, HR, m, kbeg, kend, pout_w, q);
                 });
             }
-
             // 4. backward transforms
-            const bool Mout = (op == OP_M2M);
-            double rq = Mout ? geo.rd : 1.0;  // r^(n+1) (M output) or r^-n (L output)
-            const double rqstep = Mout ? geo.rd : geo.rinvd;
-            T fo = Mout ? geo.r : AR::from_d(1.0);
-            const T qstep = Mout ? geo.r : geo.rinv;
-            for (int n = 0; n < nout_w; ++n) {
-                if (!kFF) fo = AR::from_d(rq);
-                const T f = fo;
-                const T *eo = EOUT + n * (n + 1) / 2;
-                if constexpr (FIX) {
-                    const int *WRq = p.Wq + __ldg(p.woff + n);
-                    dispatch<ACC>((n + G) / G, [&](auto na) {
-                        backward_degree_fixed<G, decltype(na)::value, ACC>(b, n, WRq, eo, f, q, tg, tq);
-                    });
-                } else {
-                    const T *WR = W + __ldg(p.woff + n);
-                    dispatch<ACC>((n + G) / G, [&](auto na) {
-                        backward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, eo, f, q, tg);
-                    });
-                }
-                if (kFF) fo = AR::mul(fo, qstep);
-                if (!kFF) rq *= rqstep;
+            f = op == OP_M2M ? geo.r : 1.0;  // r^(n+1) (M output) or r^-n (L output)
+            const T bstep = op == OP_M2M ? geo.r : geo.rinv;
+            for (int n = 0; n < pout_w; ++n) {
+                const T *WR = W + __ldg(p.woff + n);
+                dispatch<ACC>((n + G) / G, [&](auto na) {
+                    backward_degree<AR, G, decltype(na)::value, ACC>(b, n, WR, EOUT + n * (n + 1) / 2, f, q, geo.tg);
+                });
+                f *= bstep;
             }
         }
         __syncthreads();
@@ -1072,7 +925,30 @@ __device__ __forceinline__ void translate_body(const KParams &p)
                     continue;
                 }
             }
-#pragma unroll(kAccUnroll)
+            if constexpr (AR::split) {
+                // kAccBatch target loads in flight per lane; hi and lo widen by
+                // exponent re-biasing; two FP64 additions
+                if (!pid) {
+                    for (int c0 = lane; c0 < cnt; c0 += 32 * kAccBatch) {
+                        double v[kAccBatch];
+                        if (!p.atomic) {
+#pragma unroll
+                            for (int u = 0; u < kAccBatch; ++u) v[u] = c0 + 32 * u < cnt ? __ldcs(dp + c0 + 32 * u) : 0.0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < kAccBatch; ++u) {
+                            const int c = c0 + 32 * u;
+                            if (c >= cnt) continue;
+                            const T t = AR::ld(bp + c);
+                            const int e = eo * degree_at(c) + eo0;
+                            const double hd = d_from_f_scaled(t.hi, e), lo = d_from_f_scaled(t.lo, e);
+                            if (p.atomic) atomicAdd(dp + c, hd + lo);
+                            else __stcs(dp + c, (v[u] + hd) + lo);
+                        }
+                    }
+                    continue;
+                }
+            }
             for (int c = lane; c < cnt; c += 32) {
                 const int j = kScale ? degree_at(c) : 0;
                 if constexpr (AR::split) {
@@ -1124,6 +1000,16 @@ template <class A, int G, int ACC, bool HBM = true, bool WORK = false>
 __global__ void __launch_bounds__(kFxThreads, fx_blocks<A>(ACC)) k_translate_fx(KParams p)
 {
     translate_body<A, G, ACC, true, HBM, WORK>(p);
+}
+
+// resident CTAs per SM that the registers have to allow; more would spill
+// (G = 4: P=12 206 M/s with two, 166 with three)
+constexpr int split_blocks(int G, int acc) { return G == 4 ? (acc <= 2 ? 4 : acc <= 4 ? 2 : 1) : acc <= 2 ? 3 : acc == 3 ? 2 : 1; }
+// split precision
+template <int G, int ACC, bool HBM = true, bool WORK = false>
+__global__ void __launch_bounds__(256, split_blocks(G, ACC)) k_translate_split(KParams p)
+{
+    translate_body<ff, G, ACC, true, HBM, WORK>(p);
 }
 
 }  // namespace sfmm
