@@ -584,6 +584,7 @@ void sfmm_destroy(sfmm_context *c)
     }
     c->d_work.release();
     c->d_eval.release();
+    c->d_eval_grad.release();
     if (c->d_status) cudaFree(c->d_status);
     free_offsets(c);
     c->h_src.release();
@@ -851,7 +852,7 @@ int sfmm_p2x_device(sfmm_context *c, int kind, size_t nexp, size_t nq, const dou
     if (out_stride < (size_t)c->P * (c->P + 1)) return fail(c, SFMM_INVALID_ARG, "stride smaller than P(P+1)");
     cudaSetDevice(c->device);
     cudaError_t e = launch_p2x(c->dtype == SFMM_F64, kind, c->P, (long long)nexp, (long long)nq, nullptr, charge,
-                               pos, centre, out, (long long)out_stride, c->stream);
+                               pos, centre, out, (long long)out_stride, c->num_sms, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "P2M/P2L kernel");
     c->launches++;
     return SFMM_OK;
@@ -868,7 +869,7 @@ int sfmm_p2x_ragged_device(sfmm_context *c, int kind, size_t nexp, const uint32_
     if (out_stride < (size_t)c->P * (c->P + 1)) return fail(c, SFMM_INVALID_ARG, "stride smaller than P(P+1)");
     cudaSetDevice(c->device);
     cudaError_t e = launch_p2x(c->dtype == SFMM_F64, kind, c->P, (long long)nexp, 0, offset, charge, pos, centre,
-                               out, (long long)out_stride, c->stream);
+                               out, (long long)out_stride, c->num_sms, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "P2M/P2L kernel");
     c->launches++;
     return SFMM_OK;
@@ -888,20 +889,33 @@ int sfmm_eval_device(sfmm_context *c, int kind, size_t npts, const double *pos, 
     if (!box && nexp < npts) return fail(c, SFMM_INVALID_ARG, "fewer expansions than points without a box index");
     cudaSetDevice(c->device);
     // float-float normalises all nexp expansions into scratch first: worth it
-    // from one point per four expansions on.  The scratch is allocated (or
-    // grown) outside stream capture only; a call without enough of it (in a
-    // capture, or when the allocation fails) runs the FP64 kernel.
+    // from one point per four expansions on, and with the gradient's pairings
+    // beside each coefficient from four points per expansion on (P=12, 32 points
+    // each: 813 -> 720 us; one point each: level, and slower at low orders).  The scratch is allocated (or grown)
+    // outside stream capture only; a call without enough of it (in a capture,
+    // or when the allocation fails) does without the pairings, or runs the
+    // FP64 kernel.
     std::lock_guard<std::mutex> lk(c->eval_mtx);  // calls share the scratch, in stream order
     void *scratch = nullptr;
-    const size_t need = 4 * npts >= nexp ? eval_scratch_bytes(c->P, (long long)nexp) : 0;
+    bool pairings = false;
+    const size_t need = 4 * npts >= nexp ? eval_scratch_bytes(c->P, (long long)nexp, false) : 0;
     if (need) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         cudaStreamIsCapturing(c->stream, &cs);
-        if (cs == cudaStreamCaptureStatusNone && c->d_eval.ensure(need) != cudaSuccess) clear_stale_error();
-        if (c->d_eval.bytes >= need) scratch = c->d_eval.p;
+        const bool grow = cs == cudaStreamCaptureStatusNone;
+        if (gradient && npts >= 4 * nexp) {  // a buffer of its own: other calls' recorded graphs keep theirs
+            const size_t more = eval_scratch_bytes(c->P, (long long)nexp, true);
+            if (grow && c->d_eval_grad.ensure(more) != cudaSuccess) clear_stale_error();
+            pairings = c->d_eval_grad.bytes >= more;
+            if (pairings) scratch = c->d_eval_grad.p;
+        }
+        if (!scratch) {
+            if (grow && c->d_eval.ensure(need) != cudaSuccess) clear_stale_error();
+            if (c->d_eval.bytes >= need) scratch = c->d_eval.p;
+        }
     }
     cudaError_t e = launch_eval(c->dtype == SFMM_F64, kind, c->P, (long long)npts, pos, box, E, (long long)stride,
-                                (long long)nexp, centre, potential, gradient, scratch, c->stream);
+                                (long long)nexp, centre, potential, gradient, scratch, pairings, c->num_sms, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "L2P/M2P kernel");
     c->launches++;
     return SFMM_OK;

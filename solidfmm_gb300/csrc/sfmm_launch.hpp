@@ -69,15 +69,16 @@ cudaError_t launch_translate_tc(const KParams &p, const TcDevTables *t, int num_
 // expansion j takes particles [j nq, (j+1) nq), or [offset[j], offset[j+1]) with an offset array
 cudaError_t launch_p2x(bool f64, int kind, int P, long long nexp, long long nq, const uint32_t *offset,
                        const double *q, const double *pos, const double *centre, void *out, long long stride,
-                       cudaStream_t st);
+                       int num_sms, cudaStream_t st);
 
 // L2P / M2P evaluation (sfmm_p2x.cu): float-float over normalised copies of
-// the nexp expansions in `scratch` (eval_scratch_bytes of it) for orders up
-// to 32, else (scratch null or higher orders) one FP64 thread per point.
-size_t eval_scratch_bytes(int P, long long nexp);
+// the nexp expansions in `scratch` (eval_scratch_bytes of it, with the
+// gradient's pairings or without) for orders up to 32, else (scratch null or
+// higher orders) one FP64 thread per point.
+size_t eval_scratch_bytes(int P, long long nexp, bool pairings);
 cudaError_t launch_eval(bool f64, int kind, int P, long long npts, const double *pos, const uint32_t *box,
                         const void *E, long long stride, long long nexp, const double *centre, double *pot,
-                        double *grad, void *scratch, cudaStream_t st);
+                        double *grad, void *scratch, bool pairings, int num_sms, cudaStream_t st);
 
 // target[j] += slots[j] for unique host targets given by address (sfmm_p2x.cu)
 cudaError_t launch_add_slots(bool f64, long long nt, const unsigned long long *tptr, const uint32_t *cnt,

@@ -137,6 +137,10 @@ __global__ void k_p2x(int kind, int P, long long nexp, long long nq, const uint3
 // broadcast by shuffles; the diagonals v^m come from a prefix product across
 // the lanes; the harmonics accumulate in registers and are added to the
 // expansion once.
+//
+// C groups of LP lanes share an expansion, taking its charges in turn and
+// adding their sums at the end (p2x_ff_lanes chooses C): with C = 1 a warp
+// walks its 32 / LP expansions to the longest one's end.
 constexpr int kP2xColsMax = 32;
 
 // Tables, evaluated at compile time in FP64: coefficient pairs [s][m] for
@@ -281,20 +285,22 @@ __device__ __forceinline__ int max_exp3(double x, double y, double z)
 // T0 <= t < T0 + NT are added to acc[t - T0].  ab: this block's coefficient
 // table.
 template <int T0, int NT>
-__device__ __forceinline__ void p2x_columns_ff(const float4 *ab, int m1, int len1, int m2, int tot, cpx_ff dg1,
-                                               cpx_ff dg2, ff zeta, ff eta, ffacc (&ar)[NT], ffacc (&ai)[NT])
+__device__ __forceinline__ void p2x_columns_ff(const float4 *ab, int first, int m1, int len1, int m2, int tot,
+                                               cpx_ff dg1, cpx_ff dg2, ff zeta, ff eta, ffacc (&ar)[NT],
+                                               ffacc (&ai)[NT])
 {
     cpx_ff x1 = dg1, x2 = cpx_ff{ff{0.f, 0.f}, ff{0.f, 0.f}};
 #pragma unroll
     for (int t = 0; t < T0 + NT; ++t) {
         if (t >= tot) break;
         if (t > 0) {
-            const bool second = t >= len1;
+            // t < first: every lane is in its first column
+            const bool second = t >= first && t >= len1;
             const int m = second ? m2 : m1, s = second ? t - len1 : t;
             const float4 c = ab[(s > 0 ? s : 1) * kP2xColsMax + m];
             const ff A = ff_mul(ff{c.x, c.y}, zeta), B = ff_mul(ff{c.z, c.w}, eta);
             cpx_ff x = cpx_ff{ff_fms2(A, x1.r, B, x2.r), ff_fms2(A, x1.i, B, x2.i)};
-            if (s == 0) {  // the second column's diagonal
+            if (t >= first && s == 0) {  // the second column's diagonal
                 x = dg2;
                 x1 = cpx_ff{ff{0.f, 0.f}, ff{0.f, 0.f}};
             }
@@ -308,34 +314,32 @@ __device__ __forceinline__ void p2x_columns_ff(const float4 *ab, int m1, int len
     }
 }
 
-template <class Out>
-__device__ __forceinline__ void p2x_put(Out *o, int kind, int sh, int n, int m, ffacc re, ffacc im)
-{
-    const int t = n * (n + 1) / 2 + m;
-    const double f = kind == 0 ? ldexp(kP2xTab.isig[t], sh * n) : ldexp(kP2xTab.sig[t], -sh * (n + 1));
-    o[n * (n + 1) + m] += (Out)(((double)re.hi + (double)re.lo) * f);
-    o[(n + 1) * (n + 1) + m] += (Out)(((double)im.hi + (double)im.lo) * f);
-}
-
 // Harmonics T0 .. T0 + NT - 1 of every lane's run (NT = 2 LP + 1 covers all
 // of them; orders above 24 take two windows, two launches, to stay within
 // the registers).
-template <class Out, int LP, int T0, int NT>
-__global__ void __launch_bounds__(128) k_p2x_ff(int kind, int P, long long nexp, long long nq,
-                                                const uint32_t *__restrict__ offset, const double *__restrict__ q,
-                                                const double *__restrict__ pos, const double *__restrict__ centre,
-                                                Out *out, long long stride)
+// CTAs of four warps where all expansions hold the same number of charges: the
+// warps then run in step, and the unrolled harmonics (27 KB of instructions)
+// are fetched once for all of them.  CTAs of one warp where the counts differ,
+// since a CTA holds its registers until its longest expansion is done.
+constexpr int kP2xThreads = 128;
+
+template <class Out, int LP, int C, int T0, int NT>
+__global__ void __launch_bounds__(kP2xThreads) k_p2x_ff(int kind, int P, long long nexp, long long nq,
+                                                        const uint32_t *__restrict__ offset,
+                                                        const double *__restrict__ q, const double *__restrict__ pos,
+                                                        const double *__restrict__ centre, Out *out, long long stride)
 {
     __shared__ float4 ab[kP2xColsMax * kP2xColsMax];
     for (int i = threadIdx.x; i < P * kP2xColsMax; i += blockDim.x) ab[i] = (&kP2xTab.ab[0][0])[i];
     __syncthreads();
-
-    const int l = threadIdx.x % LP;
-    const long long j = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / LP;
+    constexpr int LW = LP * C;  // lanes per expansion
+    const int l = threadIdx.x % LP, gi = threadIdx.x / LP % C;
+    const long long j = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / LW;
     const bool live = j < nexp;
     const int m1 = l, m2 = P - 1 - l;  // 0 <= m2 < P
     const int len1 = (live && m1 <= m2) ? P - m1 : 0;
     const int tot = len1 + ((live && m1 < m2) ? P - m2 : 0);
+    Out *o = out + j * stride;
     long long kb = 0, cnt = 0;
     double cx = 0, cy = 0, cz = 0;
     if (live) {
@@ -344,7 +348,25 @@ __global__ void __launch_bounds__(128) k_p2x_ff(int kind, int P, long long nexp,
         cx = centre[3 * j];
         cy = centre[3 * j + 1];
         cz = centre[3 * j + 2];
+        // the expansion is read at the end
+        for (int i = threadIdx.x % LW * 128; i < P * (P + 1) * (int)sizeof(Out); i += LW * 128)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(o) + i));
     }
+    // this lane's charge of chunk c0 (the group's are c0 + gi + i C), relative
+    // to the centre; the first chunk's are kept from the pass over the exponents
+    double px = 0, py = 0, pz = 0, pq = 0;
+    auto fetch = [&](long long c0) {
+        const long long i = c0 + l * C + gi;
+        if (i < cnt) {
+            const double *pp = pos + 3 * (kb + i);
+            px = pp[0] - cx;
+            py = pp[1] - cy;
+            pz = pp[2] - cz;
+            pq = q[kb + i];
+        }
+        return i < cnt;
+    };
+    bool have = fetch(0);
     // rho = 2^sc: the largest (P2M) or smallest (P2L) distance of the
     // expansion's charges rounded to a power of two, up (P2M) or down (P2L)
     // from the components' exponents, so any double scale works: rho =
@@ -352,14 +374,17 @@ __global__ void __launch_bounds__(128) k_p2x_ff(int kind, int P, long long nexp,
     // smallest of the charges' largest components (P2L: |x'| >= 1)
     const int kNone = -(1 << 20);
     int ext = kind == 0 ? kNone : (1 << 20);
-    for (long long it = l; it < cnt; it += LP) {
-        const double *pp = pos + 3 * (kb + it);
-        const int e3 = max_exp3(pp[0] - cx, pp[1] - cy, pp[2] - cz);
+    auto extend = [&](int e3) {
         if (e3 != kNone) ext = kind == 0 ? max(ext, e3) : min(ext, e3);
+    };
+    if (have) extend(max_exp3(px, py, pz));
+    for (long long it = LW + threadIdx.x % LW; it < cnt; it += LW) {
+        const double *pp = pos + 3 * (kb + it);
+        extend(max_exp3(pp[0] - cx, pp[1] - cy, pp[2] - cz));
     }
-    for (int d = LP / 2; d > 0; d >>= 1) {
-        const int o = __shfl_xor_sync(0xffffffffu, ext, d, LP);
-        ext = kind == 0 ? max(ext, o) : min(ext, o);
+    for (int d = LW / 2; d > 0; d >>= 1) {
+        const int o2 = __shfl_xor_sync(0xffffffffu, ext, d, LW);
+        ext = kind == 0 ? max(ext, o2) : min(ext, o2);
     }
     const int sh = ext == kNone || ext == (1 << 20) ? 0 : (kind == 0 ? ext + 2 : ext);  // log2 rho
 
@@ -371,17 +396,13 @@ __global__ void __launch_bounds__(128) k_p2x_ff(int kind, int P, long long nexp,
 
     // chunk loop bound uniform over the warp (the shuffles need every lane)
     const unsigned cntw = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
-    for (unsigned c0 = 0; c0 < cntw; c0 += LP) {
-        // this lane's charge of the chunk
+    for (unsigned c0 = 0; c0 < cntw; c0 += LW) {
         ff zeta{0.f, 0.f}, eta{0.f, 0.f}, w{0.f, 0.f};
         cpx_ff v{ff{0.f, 0.f}, ff{0.f, 0.f}};
-        if (c0 + l < cnt) {
-            const long long k = kb + c0 + l;
-            const double *pp = pos + 3 * k;
-            const ff x = ff_from_d_scaled(pp[0] - cx, -sh), y = ff_from_d_scaled(pp[1] - cy, -sh),
-                     z = ff_from_d_scaled(pp[2] - cz, -sh);
+        if (have) {
+            const ff x = ff_from_d_scaled(px, -sh), y = ff_from_d_scaled(py, -sh), z = ff_from_d_scaled(pz, -sh);
             const ff r2 = ff_add(ff_add(ff_mul(x, x), ff_mul(y, y)), ff_mul(z, z));
-            w = ff_from_d_int(q[k]);
+            w = ff_from_d_int(pq);
             if (kind == 0) {
                 zeta = z;
                 eta = r2;
@@ -394,67 +415,130 @@ __global__ void __launch_bounds__(128) k_p2x_ff(int kind, int P, long long nexp,
                 w = ff_mul(w, ff_sqrt(ri));  // U_0^0 = 1/|x'|
             }
         }
-        for (int i = 0; i < LP; ++i) {
+        have = fetch(c0 + LW);  // the next chunk's loads run behind this one's arithmetic
+        const int steps = min(LP, (int)((cntw - c0 + C - 1) / C));
+#pragma unroll 1
+        for (int i = 0; i < steps; ++i) {
             const ff zi = ff_shfl(zeta, i, LP), ei = ff_shfl(eta, i, LP), wi = ff_shfl(w, i, LP);
             const cpx_ff vi = cpx_ff_shfl(v, i, LP);
             // v^l by a prefix product over the lanes; v^m2 = v^(P-LP) v^(LP-1-l)
             cpx_ff pw = l == 0 ? cpx_ff{ff{1.f, 0.f}, ff{0.f, 0.f}} : vi;
 #pragma unroll
             for (int d = 1; d < LP; d <<= 1) {
-                const cpx_ff o = cpx_ff_shfl(pw, l >= d ? l - d : l, LP);
-                if (l >= d) pw = cpx_ff_mul(pw, o);
+                const cpx_ff o2 = cpx_ff_shfl(pw, l >= d ? l - d : l, LP);
+                if (l >= d) pw = cpx_ff_mul(pw, o2);
             }
             cpx_ff ue = cpx_ff_shfl(pw, e < LP ? e : LP - 1, LP);
             if (e == LP) ue = cpx_ff_mul(ue, vi);
             const cpx_ff pm2 = cpx_ff_mul(ue, cpx_ff_shfl(pw, LP - 1 - l, LP));
             const ff k1 = ff_mul(d1, wi), k2 = ff_mul(d2, wi);
-            p2x_columns_ff<T0, NT>(ab, m1, len1, m2, tot, cpx_ff{ff_mul(pw.r, k1), ff_mul(pw.i, k1)},
-                               cpx_ff{ff_mul(pm2.r, k2), ff_mul(pm2.i, k2)}, zi, ei, ar, ai);
+            p2x_columns_ff<T0, NT>(ab, P - LP + 1, m1, len1, m2, tot,
+                                   cpx_ff{ff_mul(pw.r, k1), ff_mul(pw.i, k1)},
+                                   cpx_ff{ff_mul(pm2.r, k2), ff_mul(pm2.i, k2)}, zi, ei, ar, ai);
         }
     }
-    if (tot <= T0) return;
-    // back to R_n^m(x) = rho^n T / sig (P2M) or S_n^m(x) = sig U / rho^(n+1) (P2L)
-    Out *o = out + j * stride;
+    if constexpr (C > 1) {  // the groups' sums, the same in every group
 #pragma unroll
-    for (int u = 0; u < NT; ++u) {
-        const int t = T0 + u;
-        if (t < tot) {
-            if (t < len1) p2x_put(o, kind, sh, m1 + t, m1, ar[u], ai[u]);
-            else p2x_put(o, kind, sh, m2 + t - len1, m2, ar[u], ai[u]);
+        for (int d = LP; d < LW; d <<= 1)
+#pragma unroll
+            for (int u = 0; u < NT; ++u) {
+                ffacc_add(ar[u], ff{__shfl_xor_sync(0xffffffffu, ar[u].hi, d), __shfl_xor_sync(0xffffffffu, ar[u].lo, d)});
+                ffacc_add(ai[u], ff{__shfl_xor_sync(0xffffffffu, ai[u].hi, d), __shfl_xor_sync(0xffffffffu, ai[u].lo, d)});
+            }
+    }
+    if (tot <= T0) return;
+    // back to R_n^m(x) = rho^n T / sig (P2M) or S_n^m(x) = sig U / rho^(n+1)
+    // (P2L); group gi writes every C-th harmonic of the run, four at a time so
+    // that their loads overlap
+    constexpr int NW = (NT + C - 1) / C;
+#pragma unroll
+    for (int w0 = 0; w0 < NW; w0 += 4) {
+        double re[4], im[4];
+        Out *pr[4], *pi[4], vr[4], vi[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int u0 = (w0 + k) * C;
+            pr[k] = pi[k] = nullptr;
+            if (u0 >= NT) continue;
+            ffacc ur = ar[u0], ui = ai[u0];
+#pragma unroll
+            for (int g = 1; g < C && u0 + g < NT; ++g)
+                if (gi == g) {
+                    ur = ar[u0 + g];
+                    ui = ai[u0 + g];
+                }
+            const int t = T0 + u0 + gi;
+            if (u0 + gi < NT && t < tot) {
+                const int m = t < len1 ? m1 : m2, n = t < len1 ? m1 + t : m2 + t - len1, ix = n * (n + 1) / 2 + m;
+                const double f = kind == 0 ? ldexp(kP2xTab.isig[ix], sh * n) : ldexp(kP2xTab.sig[ix], -sh * (n + 1));
+                re[k] = ((double)ur.hi + (double)ur.lo) * f;
+                im[k] = ((double)ui.hi + (double)ui.lo) * f;
+                pr[k] = o + n * (n + 1) + m;
+                pi[k] = o + (n + 1) * (n + 1) + m;
+                vr[k] = *pr[k];
+                vi[k] = *pi[k];
+            }
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (pr[k]) {
+                *pr[k] = vr[k] + (Out)re[k];
+                *pi[k] = vi[k] + (Out)im[k];
+            }
     }
 }
 
+namespace {
+
+// orders up to 32 with LP lanes per group, C groups per expansion
+template <class Out, int LP, int C>
+void p2x_ff(int tb, int kind, int P, long long nexp, long long nq, const uint32_t *offset, const double *q,
+            const double *pos, const double *centre, Out *out, long long stride, cudaStream_t st)
+{
+    const unsigned grid = (unsigned)((nexp * LP * C + tb - 1) / tb);
+    if constexpr (LP < 16) {
+        k_p2x_ff<Out, LP, C, 0, 2 * LP + 1><<<grid, tb, 0, st>>>(kind, P, nexp, nq, offset, q, pos, centre, out, stride);
+    } else if (P <= 24) {
+        k_p2x_ff<Out, LP, C, 0, 25><<<grid, tb, 0, st>>>(kind, P, nexp, nq, offset, q, pos, centre, out, stride);
+    } else {
+        k_p2x_ff<Out, LP, C, 0, 17><<<grid, tb, 0, st>>>(kind, P, nexp, nq, offset, q, pos, centre, out, stride);
+        k_p2x_ff<Out, LP, C, 17, 16><<<grid, tb, 0, st>>>(kind, P, nexp, nq, offset, q, pos, centre, out, stride);
+    }
+}
+
+// Groups per expansion.  few: too few expansions for one group each to give
+// every scheduler half a warp; the whole warp then works on one (P=12, 64 x 32
+// charges: 62 -> 21 us).  ragged: the counts differ, and the more groups share
+// an expansion the shorter its longest neighbour makes it wait, at the price of
+// adding their sums up (32 768 expansions of 0 to 64 charges: P=8 340 us with
+// 1, 270 with 4, 285 with 8; P=12 885, 850, 1 060 with 1, 2, 4; P=24 4 260 with
+// 1, 4 610 with 2).  Otherwise one (20 000 x 32 at P=12: 318 us, 365 with 4).
+template <class Out, class... Args>
+void p2x_ff_lanes(int LP, bool few, bool ragged, Args... args)
+{
+    const int tb = few ? 32 : ragged ? (LP == 16 ? 64 : 32) : kP2xThreads;  // P=24 ragged: 4 690 us with 32, 4 595 with 64
+    switch (LP) {
+    case 1: few ? p2x_ff<Out, 1, 32>(tb, args...) : ragged ? p2x_ff<Out, 1, 4>(tb, args...) : p2x_ff<Out, 1, 1>(tb, args...); break;
+    case 2: few ? p2x_ff<Out, 2, 16>(tb, args...) : ragged ? p2x_ff<Out, 2, 4>(tb, args...) : p2x_ff<Out, 2, 1>(tb, args...); break;
+    case 4: few ? p2x_ff<Out, 4, 8>(tb, args...) : ragged ? p2x_ff<Out, 4, 4>(tb, args...) : p2x_ff<Out, 4, 1>(tb, args...); break;
+    case 8: few ? p2x_ff<Out, 8, 4>(tb, args...) : ragged ? p2x_ff<Out, 8, 2>(tb, args...) : p2x_ff<Out, 8, 1>(tb, args...); break;
+    default: few ? p2x_ff<Out, 16, 2>(tb, args...) : p2x_ff<Out, 16, 1>(tb, args...); break;
+    }
+}
+
+}  // namespace
+
 cudaError_t launch_p2x(bool f64, int kind, int P, long long nexp, long long nq, const uint32_t *offset,
                        const double *q, const double *pos, const double *centre, void *out, long long stride,
-                       cudaStream_t st)
+                       int num_sms, cudaStream_t st)
 {
     if (nexp == 0) return cudaSuccess;
     if (P <= kP2xColsMax) {  // lanes per expansion: LP <= P <= 2 LP
         const int LP = P <= 2 ? (P == 1 ? 1 : 2) : P <= 4 ? 2 : P <= 8 ? 4 : P <= 16 ? 8 : 16;
-        const int tb = 128;
-        const long long grid = (nexp * LP + tb - 1) / tb;
+        const bool ragged = offset != nullptr, few = nexp * LP < (long long)num_sms * 64 && (ragged || nq >= 4 * LP);
         clear_stale_error();
-#define SFMM_P2X_FF(T, L, T0, NT)                                                                        \
-    k_p2x_ff<T, L, T0, NT><<<(unsigned)grid, tb, 0, st>>>(kind, P, nexp, nq, offset, q, pos, centre, (T *)out, \
-                                                          stride)
-#define SFMM_P2X_LP(T)                       \
-    switch (LP) {                            \
-    case 1: SFMM_P2X_FF(T, 1, 0, 3); break;  \
-    case 2: SFMM_P2X_FF(T, 2, 0, 5); break;  \
-    case 4: SFMM_P2X_FF(T, 4, 0, 9); break;  \
-    case 8: SFMM_P2X_FF(T, 8, 0, 17); break; \
-    default:                                 \
-        if (P <= 24) {                       \
-            SFMM_P2X_FF(T, 16, 0, 25);       \
-        } else {                             \
-            SFMM_P2X_FF(T, 16, 0, 17);       \
-            SFMM_P2X_FF(T, 16, 17, 16);      \
-        }                                    \
-    }
-        if (f64) SFMM_P2X_LP(double) else SFMM_P2X_LP(float)
-#undef SFMM_P2X_LP
-#undef SFMM_P2X_FF
+        if (f64) p2x_ff_lanes<double>(LP, few, ragged, kind, P, nexp, nq, offset, q, pos, centre, (double *)out, stride, st);
+        else p2x_ff_lanes<float>(LP, few, ragged, kind, P, nexp, nq, offset, q, pos, centre, (float *)out, stride, st);
         return cudaGetLastError();
     }
     int tb = 128;
@@ -604,10 +688,55 @@ __global__ void k_eval(int kind, int P, long long npts, const double *__restrict
 __device__ __forceinline__ ff ff_of_scaled(double x, int sh) { return ff_from_d_scaled0(x, sh); }
 __device__ __forceinline__ ff ff_of_scaled(float x, int sh) { return ff{ldexp2(x, max(-252, min(252, sh))), 0.f}; }
 
-template <class In>
+// Layout of the normalised copy: entry (n, m) of an expansion at
+// eval_index(P, n, m) NS, NS = 1 (e alone) or 4 with the gradient's
+// coefficients (GRAD): e, then
+// the coefficients that T_n^m pairs with in d/dx, d/dy and d/dz, combinations
+// of the degree-(n+1) row at that row's block exponent:
+//   dx: (cp e+_re - cm e-_re, cp e+_im - cm e-_im),
+//   dy: (cp e+_im + cm e-_im, -(cp e+_re + cm e-_re)),
+//   dz: cz w_m (e0_re, e0_im),
+// e-, e0, e+ = e(n+1, m-1), e(n+1, m), e(n+1, m+1), weighted by
+// sig(n+1, m')/sig(n, m) (cm, cz, cp; at m = 0 the dx and dy pairings are
+// cp e+_re and cp e+_im).  e carries the solid dot product's weight w_m.  All
+// four sums of a point are then plain products with T_n^m.
+__device__ __forceinline__ ff ff_tab(const float2 *t, int i)
+{
+    const float2 v = t[i];
+    return ff{v.x, v.y};
+}
+__device__ __forceinline__ float4 eval_pack(ff r, ff i, float w) { return make_float4(r.hi * w, r.lo * w, i.hi * w, i.lo * w); }
+// the three pairings of T_n^m (index ix = n(n+1)/2 + m) from the unweighted
+// entries m - 1, m, m + 1 of degree n + 1
+__device__ __forceinline__ void eval_pairings(int ix, int m, cpx_ff em, cpx_ff e0, cpx_ff ep, float4 *g)
+{
+    using A = arith<ff>;
+    const ff cp = ff_tab(kP2xTab.cp, ix), cm = ff_tab(kP2xTab.cm, ix), cz = ff_tab(kP2xTab.cz, ix);
+    if (m == 0) {
+        const ff zero{0.f, 0.f};
+        g[0] = eval_pack(ff_mul(cp, ep.r), zero, 1.f);
+        g[1] = eval_pack(ff_mul(cp, ep.i), zero, 1.f);
+    } else {
+        const ff ncm = A::neg(cm);
+        g[0] = eval_pack(A::dot2(cp, ep.r, ncm, em.r), A::dot2(cp, ep.i, ncm, em.i), 1.f);
+        g[1] = eval_pack(A::dot2(cp, ep.i, cm, em.i), A::neg(A::dot2(cp, ep.r, cm, em.r)), 1.f);
+    }
+    g[2] = eval_pack(ff_mul(cz, e0.r), ff_mul(cz, e0.i), m ? 2.f : 1.f);
+}
+
+// entry (n, m) of the copy: column by column, so that a point's walk along a
+// column reads consecutive entries
+__device__ __forceinline__ int eval_index(int P, int n, int m) { return m * P - m * (m - 1) / 2 + n - m; }
+
+// One thread per expansion and degree n; with pairings also those of degree
+// n - 1, from this row's entries.  (A warp per expansion, with coalesced stores
+// but 450 instructions per 32 coefficients, took as long at P=12 and half as
+// long again at P=4 and 8.)
+template <class In, bool GRAD>
 __global__ void k_eval_prep(int kind, int P, long long nexp, const In *__restrict__ E, long long stride,
                             float4 *__restrict__ Mout, int *__restrict__ sdeg)
 {
+    constexpr int NS = GRAD ? 4 : 1;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= nexp * P) return;
     const long long b = i / P;
@@ -615,44 +744,67 @@ __global__ void k_eval_prep(int kind, int P, long long nexp, const In *__restric
     const In *e = E + b * stride;
     const int t0 = n * (n + 1) / 2;
     int s = -(1 << 20);
+#pragma unroll 4
     for (int m = 0; m <= n; ++m) {
         const int se = kind ? kP2xTab.se[t0 + m] : -kP2xTab.se[t0 + m];
         s = max(s, max(exp_of(e[n * (n + 1) + m]), exp_of(e[(n + 1) * (n + 1) + m])) + se);
     }
     sdeg[i] = s;  // an all-zero degree keeps -2^20: it never sets a point's scale
-    float4 *o = Mout + b * (P * (P + 1) / 2) + t0;
-    for (int m = 0; m <= n; ++m) {
+    float4 *o = Mout + b * (P * (P + 1) / 2) * NS;
+    auto coef = [&](int m) {
         const int se = kind ? kP2xTab.se[t0 + m] : -kP2xTab.se[t0 + m];
-        const float2 f2 = kind ? kP2xTab.fs[t0 + m] : kP2xTab.fi[t0 + m];
-        const ff f{f2.x, f2.y};
-        const ff re = ff_mul(ff_of_scaled(e[n * (n + 1) + m], se - s), f);
-        const ff im = ff_mul(ff_of_scaled(e[(n + 1) * (n + 1) + m], se - s), f);
-        o[m] = make_float4(re.hi, re.lo, im.hi, im.lo);
+        const ff f = kind ? ff_tab(kP2xTab.fs, t0 + m) : ff_tab(kP2xTab.fi, t0 + m);
+        return cpx_ff{ff_mul(ff_of_scaled(e[n * (n + 1) + m], se - s), f),
+                      ff_mul(ff_of_scaled(e[(n + 1) * (n + 1) + m], se - s), f)};
+    };
+    cpx_ff em{}, e0 = coef(0);
+    for (int m = 0; m <= n; ++m) {
+        const cpx_ff ep = GRAD && m < n ? coef(m + 1) : cpx_ff{};
+        o[eval_index(P, n, m) * NS] = eval_pack(e0.r, e0.i, m ? 2.f : 1.f);
+        if constexpr (GRAD) {
+            if (m < n) eval_pairings(t0 - n + m, m, em, e0, ep, o + eval_index(P, n - 1, m) * NS + 1);
+            if (n == P - 1)  // no degree above
+                for (int k = 1; k < 4; ++k) o[eval_index(P, n, m) * NS + k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            em = e0;
+            e0 = ep;
+        } else if (m < n) {
+            e0 = coef(m + 1);
+        }
     }
 }
 
-// coefficient (n, m) of expansion row Mb times 2^ex (|M| < 4: beyond +-252
-// the product under- or overflows FP32 in any case)
-__device__ __forceinline__ cpx_ff eval_coef(const float4 *Mb, int n, int m, int ex)
-{
-    ex = max(-252, min(252, ex));
-    const float4 v = __ldg(Mb + n * (n + 1) / 2 + m);
-    return cpx_ff{ff{ldexp2(v.x, ex), ldexp2(v.y, ex)}, ff{ldexp2(v.z, ex), ldexp2(v.w, ex)}};
-}
-__device__ __forceinline__ ff ff_tab(const float2 *t, int i)
-{
-    const float2 v = t[i];
-    return ff{v.x, v.y};
-}
-__device__ __forceinline__ void ffacc_madd(ffacc &a, ff w, ff x) { ffacc_add(a, ff_mul(w, x)); }
+// a float-float value times 2^ex (ex <= 0, beyond -252 it vanishes in any case) by the factors f1, f2
+struct ff_scale {
+    float f1, f2;
+    __device__ __forceinline__ explicit ff_scale(int ex)
+    {
+        ex = max(-252, min(252, ex));
+        f1 = pow2f(ex / 2);
+        f2 = pow2f(ex - ex / 2);
+    }
+    __device__ __forceinline__ ff operator()(ff v) const { return ff{__fmul_rn(__fmul_rn(v.hi, f1), f2), __fmul_rn(__fmul_rn(v.lo, f1), f2)}; }
+};
+// How a point's gradient is formed: not at all, from the prepared pairings
+// (half the work per point, 110 more operations per coefficient of every
+// expansion: from four points per expansion on), or from e itself.
+enum { GRAD_NONE = 0, GRAD_PREPARED = 1, GRAD_DIRECT = 2 };
 
+// C lanes per point, the columns m dealt to them back and forth (their
+// lengths fall by one per column).  One lane per point keeps every lane busy;
+// with few points the rest of the GPU is idle, and four finish a point sooner.
+template <int GRAD, int C>
 __global__ void __launch_bounds__(128) k_eval_ff(int kind, int P, long long npts, const double *__restrict__ pos,
                                                  const uint32_t *__restrict__ box, const float4 *__restrict__ M,
                                                  const int *__restrict__ sdeg, const double *__restrict__ centre,
                                                  double *pot, double *grad)
 {
-    const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (j >= npts) return;
+    using A = arith<ff>;
+    constexpr int NS = GRAD == GRAD_PREPARED ? 4 : 1, NT = GRAD ? 4 : 1;
+    const long long jt = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / C;
+    if (C == 1 && jt >= npts) return;
+    const bool live = jt < npts;
+    const long long j = live ? jt : npts - 1;  // the lanes of a point finish together
+    const int lane = threadIdx.x % C;
     const long long b = box ? (long long)box[j] : j;
     const double dx = pos[3 * j] - centre[3 * b], dy = pos[3 * j + 1] - centre[3 * b + 1],
                  dz = pos[3 * j + 2] - centre[3 * b + 2];
@@ -675,9 +827,8 @@ __global__ void __launch_bounds__(128) k_eval_ff(int kind, int P, long long npts
         v = cpx_ff{ff_mul(x, ri), ff_mul(y, ri)};
         w0 = ff_sqrt(ri);  // U_0^0 = 1/|x'|
     }
-    const float4 *Mb = M + b * (P * (P + 1) / 2);
+    const float4 *Mb = M + b * (P * (P + 1) / 2) * NS;
     const int *sb = sdeg + b * P;
-    const bool want_grad = grad != nullptr && kind == 0;
     // the sums run at the scale 2^-B of the largest degree and return to
     // their own in FP64, so results beyond the FP32 range keep their digits
     int B = -(1 << 29);
@@ -691,75 +842,126 @@ __global__ void __launch_bounds__(128) k_eval_ff(int kind, int P, long long npts
     for (int i = 1; i < 5; ++i) v2i[i] = cpx_ff_mul(v2i[i - 1], v2i[i - 1]);
     // each column sums into fresh accumulators (at most P terms), added to
     // the totals with a renormalising float-float addition
-    ff phi{0.f, 0.f}, gx{0.f, 0.f}, gy{0.f, 0.f}, gz{0.f, 0.f};
-    for (int m = 0; m < P; ++m) {
+    ff tot[NT];
+#pragma unroll
+    for (int k = 0; k < NT; ++k) tot[k] = ff{0.f, 0.f};
+    for (int m0 = 0, back = 0; m0 < P; m0 += C, back ^= 1) {
+        const int m = m0 + (back ? C - 1 - lane : lane);
+        if (m >= P) continue;
         cpx_ff vm{w0, ff{0.f, 0.f}};  // v^m / |x'| (M2P) or v^m (L2P)
 #pragma unroll
         for (int i = 0; i < 5; ++i)
             if (m >> i & 1) vm = cpx_ff_mul(vm, v2i[i]);
         const ff dm = ff_tab(kP2xTab.diag, m);
         cpx_ff x1{ff_mul(dm, vm.r), ff_mul(dm, vm.i)}, x2{ff{0.f, 0.f}, ff{0.f, 0.f}};
-        ffacc cphi{0.f, 0.f}, cgx{0.f, 0.f}, cgy{0.f, 0.f}, cgz{0.f, 0.f};
-        const float wm = m ? 2.f : 1.f;
-        for (int n = m; n < P; ++n) {
+        ffacc acc[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) acc[k] = ffacc{0.f, 0.f};
+        // exponent of degree n and the factors that apply it to T_n^m
+        auto entry = [](float4 v, bool weighted) {  // e without its weight
+            const float h = weighted ? 0.5f : 1.f;
+            return cpx_ff{ff{v.x * h, v.y * h}, ff{v.z * h, v.w * h}};
+        };
+        auto exponent = [&](int n) { return (kind == 0 ? sb[n] + n * sh : sb[n] - (n + 1) * sh) - B; };
+        ff_scale s0(exponent(m));
+        const float4 *e = Mb + eval_index(P, m, m) * NS;
+        // the columns beside this one, at the same degree
+        const float4 *left = Mb + (m ? eval_index(P, m, m - 1) : 0) * NS, *right = Mb + eval_index(P, m, m + 1) * NS;
+#pragma unroll 2
+        for (int n = m; n < P; ++n, e += NS) {
             if (n > m) {
                 const float4 c = kP2xTab.ab[n - m][m];
-                const ff A = ff_mul(ff{c.x, c.y}, zeta), B = ff_mul(ff{c.z, c.w}, eta);
-                const cpx_ff xn{ff_fms2(A, x1.r, B, x2.r), ff_fms2(A, x1.i, B, x2.i)};
+                const ff a = ff_mul(ff{c.x, c.y}, zeta), bb = ff_mul(ff{c.z, c.w}, eta);
+                const cpx_ff xn{ff_fms2(a, x1.r, bb, x2.r), ff_fms2(a, x1.i, bb, x2.i)};
                 x2 = x1;
                 x1 = xn;
             }
-            const int ex = (kind == 0 ? sb[n] + n * sh : sb[n] - (n + 1) * sh) - B;
-            const cpx_ff e = eval_coef(Mb, n, m, ex);
-            const ff t = ff_fms2(e.r, x1.r, ff{-e.i.hi, -e.i.lo}, x1.i);  // e_re X_re + e_im X_im
-            ffacc_add(cphi, ff{t.hi * wm, t.lo * wm});
-            if (want_grad && n + 1 < P) {
-                const int k1 = n + 1, ix = n * (n + 1) / 2 + m, ex1 = sb[k1] + k1 * sh - B;
-                const cpx_ff ez = eval_coef(Mb, k1, m, ex1);
-                const ff tz = ff_fms2(ez.r, x1.r, ff{-ez.i.hi, -ez.i.lo}, x1.i);
-                ffacc_madd(cgz, ff_tab(kP2xTab.cz, ix), ff{tz.hi * wm, tz.lo * wm});
-                const cpx_ff ep = eval_coef(Mb, k1, m + 1, ex1);
-                const ff cp = ff_tab(kP2xTab.cp, ix);
-                if (m == 0) {  // R_k^0 is real
-                    ffacc_madd(cgx, cp, ff_mul(x1.r, ep.r));
-                    ffacc_madd(cgy, cp, ff_mul(x1.r, ep.i));
-                } else {
-                    const cpx_ff em = eval_coef(Mb, k1, m - 1, ex1);
-                    const ff cm = ff_tab(kP2xTab.cm, ix);
-                    // conj(R) (L^{m+1} - L^{m-1}) and conj(R) (L^{m-1} + L^{m+1}), each L weighted
-                    const ff xr = ff_fms2(cp, ep.r, cm, em.r), xi = ff_fms2(cp, ep.i, cm, em.i);
-                    const ff yr = ff_fms2(cm, em.r, ff{-cp.hi, -cp.lo}, ep.r);
-                    const ff yi = ff_fms2(cm, em.i, ff{-cp.hi, -cp.lo}, ep.i);
-                    ffacc_add(cgx, ff_fms2(x1.r, xr, ff{-x1.i.hi, -x1.i.lo}, xi));
-                    ffacc_add(cgy, ff_fms2(x1.r, yi, x1.i, yr));
+            auto add = [&](ffacc &t, const float4 c, cpx_ff u) {
+                A::mac(t, ff{c.x, c.y}, u.r);
+                if (m) A::mac(t, ff{c.z, c.w}, u.i);  // real at m = 0
+            };
+            add(acc[0], __ldg(e), cpx_ff{s0(x1.r), s0(x1.i)});
+            if (n + 1 < P) {
+                s0 = ff_scale(exponent(n + 1));
+                if constexpr (GRAD != GRAD_NONE) {
+                    const cpx_ff u{s0(x1.r), s0(x1.i)};
+                    float4 g[3];
+                    if constexpr (GRAD == GRAD_PREPARED) {
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) g[k] = __ldg(e + k + 1);
+                    } else {
+                        const int up = n + 1 - m;
+                        eval_pairings(n * (n + 1) / 2 + m, m, m ? entry(__ldg(left + up), m > 1) : cpx_ff{},
+                                      entry(__ldg(e + 1), m > 0), entry(__ldg(right + up), true), g);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) add(acc[k + 1], g[k], u);
                 }
             }
         }
-        phi = ff_add(phi, ff{cphi.hi, cphi.lo});
-        if (want_grad) {
-            gx = ff_add(gx, ff{cgx.hi, cgx.lo});
-            gy = ff_add(gy, ff{cgy.hi, cgy.lo});
-            gz = ff_add(gz, ff{cgz.hi, cgz.lo});
-        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) tot[k] = ff_add(tot[k], A::fin(acc[k]));
     }
-    pot[j] += ldexp((double)phi.hi + (double)phi.lo, B);
-    if (want_grad) {
+#pragma unroll
+    for (int d = 1; d < C; d <<= 1)
+#pragma unroll
+        for (int k = 0; k < NT; ++k)
+            tot[k] = ff_add(tot[k], ff{__shfl_xor_sync(0xffffffffu, tot[k].hi, d), __shfl_xor_sync(0xffffffffu, tot[k].lo, d)});
+    if (!live || lane) return;
+    pot[j] += ldexp((double)tot[0].hi + (double)tot[0].lo, B);
+    if constexpr (GRAD != GRAD_NONE) {
         const double ir = ldexp(1.0, B - sh);
-        grad[3 * j] += ((double)gx.hi + (double)gx.lo) * ir;
-        grad[3 * j + 1] += ((double)gy.hi + (double)gy.lo) * ir;
-        grad[3 * j + 2] += ((double)gz.hi + (double)gz.lo) * ir;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) grad[3 * j + k] += ((double)tot[k + 1].hi + (double)tot[k + 1].lo) * ir;
     }
 }
 
-size_t eval_scratch_bytes(int P, long long nexp)
+// scratch of the normalised copy, with or without the gradient's pairings
+size_t eval_scratch_bytes(int P, long long nexp, bool pairings)
 {
     if (P > kP2xColsMax) return 0;
-    return (size_t)nexp * ((size_t)P * (P + 1) / 2 * sizeof(float4) + (size_t)P * sizeof(int));
+    return (size_t)nexp * ((size_t)P * (P + 1) / 2 * (pairings ? 4 : 1) * sizeof(float4) + (size_t)P * sizeof(int));
 }
+
+namespace {
+
+struct EvalArgs {
+    int kind, P;
+    long long npts;
+    const double *pos;
+    const uint32_t *box;
+    const float4 *M;
+    const int *sdeg;
+    const double *centre;
+    double *pot, *grad;
+};
+
+template <int GRAD>
+void eval_points(const EvalArgs &a, bool few, cudaStream_t st)
+{
+    const int tb = 128, C = few ? 4 : 1;
+    const unsigned grid = (unsigned)((a.npts * C + tb - 1) / tb);
+    if (few)
+        k_eval_ff<GRAD, 4><<<grid, tb, 0, st>>>(a.kind, a.P, a.npts, a.pos, a.box, a.M, a.sdeg, a.centre, a.pot, a.grad);
+    else
+        k_eval_ff<GRAD, 1><<<grid, tb, 0, st>>>(a.kind, a.P, a.npts, a.pos, a.box, a.M, a.sdeg, a.centre, a.pot, a.grad);
+}
+
+template <class In>
+void eval_prep(int kind, int P, long long nexp, const void *E, long long stride, float4 *M, int *sdeg, bool pairings,
+               cudaStream_t st)
+{
+    const int tb = 128;
+    const unsigned gp = (unsigned)((nexp * P + tb - 1) / tb);
+    if (pairings) k_eval_prep<In, true><<<gp, tb, 0, st>>>(kind, P, nexp, (const In *)E, stride, M, sdeg);
+    else k_eval_prep<In, false><<<gp, tb, 0, st>>>(kind, P, nexp, (const In *)E, stride, M, sdeg);
+}
+
+}  // namespace
 
 cudaError_t launch_eval(bool f64, int kind, int P, long long npts, const double *pos, const uint32_t *box,
                         const void *E, long long stride, long long nexp, const double *centre, double *pot,
-                        double *grad, void *scratch, cudaStream_t st)
+                        double *grad, void *scratch, bool pairings, int num_sms, cudaStream_t st)
 {
     if (npts == 0) return cudaSuccess;
     const int tb = 128;
@@ -767,13 +969,15 @@ cudaError_t launch_eval(bool f64, int kind, int P, long long npts, const double 
     clear_stale_error();
     if (scratch && P <= kP2xColsMax) {  // float-float: normalise every expansion once, then the points
         float4 *Mn = static_cast<float4 *>(scratch);
-        int *sdeg = reinterpret_cast<int *>(Mn + (size_t)nexp * (P * (P + 1) / 2));
-        const long long gp = (nexp * P + tb - 1) / tb;
-        if (f64)
-            k_eval_prep<double><<<(unsigned)gp, tb, 0, st>>>(kind, P, nexp, (const double *)E, stride, Mn, sdeg);
-        else
-            k_eval_prep<float><<<(unsigned)gp, tb, 0, st>>>(kind, P, nexp, (const float *)E, stride, Mn, sdeg);
-        k_eval_ff<<<(unsigned)grid, tb, 0, st>>>(kind, P, npts, pos, box, Mn, sdeg, centre, pot, grad);
+        const size_t entries = (size_t)nexp * (P * (P + 1) / 2) * (pairings ? 4 : 1);
+        int *sdeg = reinterpret_cast<int *>(Mn + entries);
+        if (f64) eval_prep<double>(kind, P, nexp, E, stride, Mn, sdeg, pairings, st);
+        else eval_prep<float>(kind, P, nexp, E, stride, Mn, sdeg, pairings, st);
+        const EvalArgs a{kind, P, npts, pos, box, Mn, sdeg, centre, pot, grad};
+        const bool few = npts < (long long)num_sms * 256;
+        if (!grad || kind != 0) eval_points<GRAD_NONE>(a, few, st);
+        else if (pairings) eval_points<GRAD_PREPARED>(a, few, st);
+        else eval_points<GRAD_DIRECT>(a, few, st);
         return cudaGetLastError();
     }
     if (f64)
