@@ -21,8 +21,9 @@
 // the FP64 pipe to the z-translation, whose coefficients span too many orders of
 // magnitude for a block exponent, and to the accumulation into the targets.
 // Measured (M2L, one GB300): P=16 37.1 -> 86.9 M/s, P=8 168 -> 387, P=24 11.7
-// -> 25.2, with an error no larger than the FP64 transforms' (3.2e-15 against
-// 3.5e-15 of a P=16 batch).  What bounds it now: the FP64 pipe is busy 55% of
+// -> 25.2, with an error no larger than the FP64 transforms' (P=16 M2L 2.1e-15
+// against 3.4e-15, M2M 7.1e-17 against 9.1e-17, P=21 L2L 2e-16 against 4.5e-15).
+// What bounds it now: the FP64 pipe is busy 55% of
 // the time with the z-translation alone, the schedulers issue in 45% of the
 // cycles with 20 resident warps (registers and shared memory).
 //
@@ -178,6 +179,20 @@ struct FxTrig {
     fx ca[ACC], sa[ACC], cb[ACC], sb[ACC];
 };
 
+// (c, s) of unit length but for the roundings of two doubles, made one to a few
+// units of 2^-60.  A translation rotates back what it rotated forth, so the
+// error in length of (c, s) enters element m of its result m times over; the
+// angle's own rounding mostly cancels.
+__device__ __forceinline__ void fx_unit(long long &c, long long &s)
+{
+    const fx cl = fx_split_centred(c + (1 << 29)), sl = fx_split_centred(s + (1 << 29));
+    const long long d = fx_dot2(cl, cl, sl, sl) - (1ll << 60);  // c^2 + s^2 - 1
+    if (d > -(1 << 20) && d < (1 << 20)) {
+        c -= mul_wide(cl.h, (int)d) >> 31;
+        s -= mul_wide(sl.h, (int)d) >> 31;
+    }
+}
+
 // Per-translation geometry, computed once per tile by one thread each.
 // From the shift (already negated for M2M).  The components are scaled by a
 // power of two first, so that squares neither overflow nor underflow.
@@ -199,12 +214,21 @@ __device__ __forceinline__ void fx_geometry(double x, double y, double z, FxGeo 
     g.sa = fx_q60(sa);
     g.cb = fx_q60(zs * rinv);
     g.sb = fx_q60(-rxy * rinv);
+    fx_unit(g.ca, g.sa);
+    fx_unit(g.cb, g.sb);
     const fxd vr = fx_unpack(r), vi = fx_unpack(rinv);
     g.r = fx_word(vr);
     g.rinv = fx_word(vi);
     g.re = vr.eb - 1022 + k;
     g.rinve = vi.eb - 1022 - k;
     if (!(r > 0.0) || !isfinite(r)) g.re = g.rinve = kFxBad;
+    else {
+        // r / r = 1 to 2^-59 instead of 2^-53: M2M and L2L multiply by r^n and
+        // r^-n.  r is in [1, 4), so the words' product is 1 / 2 or 1 / 4.
+        const int e = vr.eb + vi.eb - 2044;
+        const long long d = fx_mul(fx_split(g.r), fx_split(g.rinv)) - (1ll << (60 - e));
+        g.rinv = max(g.rinv - (mul_wide((int)(g.rinv >> 30), (int)d) >> (30 - e)), 1ll << 59);
+    }
     *out = g;
 }
 
