@@ -311,12 +311,19 @@ __device__ __forceinline__ void swap_fx(const int2 *__restrict__ W, const double
 __device__ __forceinline__ int fx_headroom(int d) { return d <= 2 ? 1 : d <= 8 ? 2 : d <= 32 ? 3 : 4; }
 
 // one row: doubles from the mantissas M 2^E (NaN for a bad row); safe: every
-// exponent is far from the ends of the FP64 range
+// exponent is far from the ends of the FP64 range.  Zeros need no exponent:
+// the rows above a source's own order take the fast form too.
 template <int G, int NA>
 __device__ __forceinline__ void fx_store_row(double *own, int d, int r, const long long (&M)[NA], const int (&E)[NA],
                                              bool safe, bool bad)
 {
     constexpr int RS = G / 2;
+    if (!safe) {
+        long long any = 0;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) any |= M[a];
+        safe = any == 0;
+    }
     if (safe && !bad) {
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
