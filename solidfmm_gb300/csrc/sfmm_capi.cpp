@@ -458,18 +458,20 @@ LaunchShape best_shape(Arith a, int P, int G, bool small_tiles, int min_threads)
     // (split M2L P=22: 1 976 CTAs of 32 threads, instruction-fetch stalls and
     // a lower L1 hit rate for the tables); smaller CTAs when no larger tile
     // fits, or when sfmm_tune measures them faster (split P=27: +6%).  The
-    // 60-bit kernel also takes three warps where they hold an eighth more
-    // threads: M2L P=24 20.4 -> 22.3 M/s, P=30 8.3 -> 11.1, while with fewer
-    // (P=20) or equal numbers four win (47.7 against 42.0).  One- and two-warp
-    // CTAs would give P=24 25.3 and 24.0 and P=21 37.7 (33.2), but only while
-    // all of them run in step: on a launch of orders 4 to 24 in no order they
-    // wait for instructions (9.1 and 14.7 M/s; three warps 20.3, four 22.5).
+    // 60-bit kernel also takes two warps (three above order 22) where they
+    // hold an eighth more threads: M2L P=21 33.2 -> 37.7 M/s, P=24 20.4 ->
+    // 22.3, P=30 8.3 -> 11.1, while with fewer (P=20) or equal numbers four win
+    // (47.7 against 42.0).  One- and two-warp CTAs would give P=24 25.3 and
+    // 24.0, but only while all of them run in step: on a launch of orders 4 to
+    // 24 in no order they wait for instructions (9.1 and 14.7 M/s; three warps
+    // 20.3, four 22.5), which up to order 22 costs nothing (32.5 against 32.4).
+    const int few = a == Arith::F64 ? (P <= 22 ? 64 : 96) : 32;
     LaunchShape best[2];
     long most[2] = {0, 0};
     for (int k = 0; k < 2; ++k)
         for (int ts = 256 / G; ts >= 32 / G; ts -= 32 / G) {
             LaunchShape s = translate_shape(a, P, G, ts);
-            if (!s.acc || s.threads < (k ? (a == Arith::F64 && best[0].acc ? 96 : 32) : min_threads)) continue;
+            if (!s.acc || s.threads < (k ? (best[0].acc ? few : 32) : min_threads)) continue;
             s.blocks_per_sm = translate_blocks_per_sm(a, s);
             const long th = (long)s.blocks_per_sm * s.threads;
             if (th > 0 && (th > most[k] || (small_tiles && th == most[k]))) {
