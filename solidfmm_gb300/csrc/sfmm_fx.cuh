@@ -195,19 +195,22 @@ __device__ __forceinline__ void fx_unit(long long &c, long long &s)
 
 // Per-translation geometry, computed once per tile by one thread each.
 // From the shift (already negated for M2M).  The components are scaled by a
-// power of two first, so that squares neither overflow nor underflow.
+// power of two first, so that squares neither overflow nor underflow; the
+// transverse ones by their own, since (cos, sin) of the azimuth are as long as
+// 1 only while no square underflows beside a far larger z.
 __device__ __forceinline__ void fx_geometry(double x, double y, double z, FxGeo *out)
 {
-    const int k = max(exp_of(x), max(exp_of(y), exp_of(z)));
-    const double xs = d_scaled(x, -k), ys = d_scaled(y, -k), zs = d_scaled(z, -k);
-    const double rxy2 = fma(xs, xs, ys * ys);
-    const double r = sqrt(fma(zs, zs, rxy2)), rxy = sqrt(rxy2);
+    const int ka = max(exp_of(x), exp_of(y)), k = max(ka, exp_of(z));
+    const double xa = d_scaled(x, -ka), ya = d_scaled(y, -ka), zs = d_scaled(z, -k);
+    const double ra2 = fma(xa, xa, ya * ya), ra = sqrt(ra2);
+    const double rxy = d_scaled(ra, ka - k);
+    const double r = sqrt(fma(zs, zs, d_scaled(ra2, 2 * (ka - k))));
     const double rinv = 1.0 / r;
     double ca = 1.0, sa = 0.0;
-    if (rxy > 0) {
-        const double ri = 1.0 / rxy;
-        ca = ys * ri;
-        sa = xs * ri;
+    if (ra > 0) {
+        const double ri = 1.0 / ra;
+        ca = ya * ri;
+        sa = xa * ri;
     }
     FxGeo g;
     g.ca = fx_q60(ca);
