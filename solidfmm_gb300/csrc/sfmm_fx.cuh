@@ -348,13 +348,56 @@ __device__ __forceinline__ void fx_store_row(double *own, int d, int r, const lo
     }
 }
 
+// Rows next to the smallest doubles.  Subnormals have fewer bits than their
+// exponent says, and an edge factor (2^-142 to 2^142) may raise them to any
+// size; a zero counts with the exponent 1 and its edge factor's.  Neither
+// reaches the block exponent of a row whose largest element has a biased
+// exponent above kFxTiny.  The gather looks for coefficients up to there, and
+// takes rows that have no larger one times 2^kFxRaise.
+constexpr int kFxTiny = 406;
+constexpr int kFxRaise = 600;
+// The running minimum over coefficients that finds them: the high word less
+// one, zeros above all others.
+__device__ __forceinline__ unsigned fx_low(double x, unsigned low)
+{
+    return min(low, (((unsigned)__double2hiint(x) & 0x7fffffffu) | min((unsigned)__double2loint(x), 1u)) - 1u);
+}
+__device__ __forceinline__ bool fx_tiny(unsigned low) { return low < (unsigned)(kFxTiny + 1) << 20; }
+// The degrees raised are noted in the last word of the buffer's padding, which
+// the swaps multiply by zero coefficients only.
+__device__ __forceinline__ int fx_raised(const double *b, int spad, int n)
+{
+    return *reinterpret_cast<const unsigned *>(b + spad - 1) >> n & 1u ? kFxRaise : 0;
+}
+// One expansion of order P by one warp.
+__device__ __forceinline__ void fx_raise_rows(double *b, int spad, int P, int lane)
+{
+    unsigned raised = 0;
+    __syncwarp();
+#pragma unroll 1
+    for (int n = 0; n < P; ++n) {
+        const int d = n + 1;
+        double *row = b + n * d;
+        int top = kFxNone;
+        for (int c = lane; c < 2 * d; c += 32) {
+            const fxd x = fx_unpack(c == d ? 0.0 : row[c]);  // the imaginary part at m = 0 is zero
+            if (x.mh | x.ml) top = max(top, x.eb);
+        }
+        top = group_max_int<32>(top);
+        if (top == kFxNone || top > kFxTiny) continue;
+        for (int c = lane; c < 2 * d; c += 32) row[c] *= __hiloint2double((1023 + kFxRaise) << 20, 0);
+        raised |= 1u << n;
+    }
+    if (lane == 0) *reinterpret_cast<unsigned *>(b + spad - 1) = raised;
+}
+
 // One degree of the forward transform: edge (r-power and basis factor g, one
 // product per element), rotation by alpha, swap, rotation by beta, swap;
 // doubles in, doubles out.
 template <int G, int NA, int ACC>
 __device__ __forceinline__ void forward_degree_fx(double *b, int n, const int2 *__restrict__ W,
-                                                  const int4 *__restrict__ ein, fxs f, bool bad, int q,
-                                                  const FxTrig<ACC> &tg)
+                                                  const int4 *__restrict__ ein, fxs f, bool bad, int spad,
+                                                  int q, const FxTrig<ACC> &tg)
 {
     constexpr int RS = G / 2;
     const int d = n + 1, r = q >> 1, part = q & 1, j0 = (r + n + part) & 1, cnt = (d + 1) >> 1;
@@ -400,7 +443,7 @@ __device__ __forceinline__ void forward_degree_fx(double *b, int n, const int2 *
     __syncwarp();
     swap_fx<G, NA>(W, own, j0, cnt, q, kFxRound, M);
     __syncwarp();
-    const int E = emax + f.e - 1022 - 60 + hb;
+    const int E = emax + f.e - 1022 - 60 + hb - fx_raised(b, spad, n);
     int Ea[NA];
 #pragma unroll
     for (int a = 0; a < NA; ++a) Ea[a] = E;

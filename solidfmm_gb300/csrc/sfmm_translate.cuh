@@ -638,6 +638,7 @@ __device__ __forceinline__ void translate_body(const KParams &p)
         //    slots past a row and multiply them by zero coefficients).
         //    Sources and targets stream through with evict-first hints so the
         //    coefficient tables stay in the L1 left beside the buffers.
+        [[maybe_unused]] unsigned low = 0xffffffffu;
         for (int s = warp; s < TS; s += nwarps) {
             const int ps = (int)(m_pin[s] & 0xffffu);
             const int cnt = ps * (ps + 1);
@@ -662,15 +663,25 @@ __device__ __forceinline__ void translate_body(const KParams &p)
                 for (int c = lane; c < p.spad; c += 32)
                     AR::st(bp + c, c < cnt ? src_scaled(__ldcs(sp + c), es * degree_at(c) + e0, (const T *)nullptr)
                                            : AR::zero());
-            } else if constexpr (HBM) {  // kGatherUnroll loads in flight per lane
-#pragma unroll(kGatherUnroll)
-                for (int c = lane; c < p.spad; c += 32)
-                    AR::st(bp + c, c < cnt ? AR::from_src(__ldcs(sp + c)) : AR::zero());
             } else {
-                for (int c = lane; c < p.spad; c += 32)
-                    AR::st(bp + c, c < cnt ? AR::from_src(__ldcs(sp + c)) : AR::zero());
+                auto put = [&](int c) {
+                    const Src v = c < cnt ? __ldcs(sp + c) : Src(0);
+                    if constexpr (PL && !F32) low = fx_low(v, low);
+                    AR::st(bp + c, AR::from_src(v));
+                };
+                if constexpr (HBM) {  // kGatherUnroll loads in flight per lane
+#pragma unroll(kGatherUnroll)
+                    for (int c = lane; c < p.spad; c += 32) put(c);
+                } else {
+                    for (int c = lane; c < p.spad; c += 32) put(c);
+                }
             }
         }
+        if constexpr (PL && !F32)
+            if (__any_sync(FULL, fx_tiny(low)))
+#pragma unroll 1
+                for (int s = warp; s < TS; s += nwarps)
+                    fx_raise_rows(buf0 + (long long)s * p.spad, p.spad, (int)(m_pin[s] & 0xffffu), lane);
         // A tile of more than one pair of orders runs all its warps to the
         // tile's largest: they wait for each other at its end anyway, and in
         // step they share the instruction cache, which holds a part of the
@@ -791,7 +802,7 @@ __device__ __forceinline__ void translate_body(const KParams &p)
             const int4 *e = EIN;
             for_degrees<ACC, G / 2>(pin_w, [&](auto na, int n) {
                 constexpr int NA = decltype(na)::value;
-                forward_degree_fx<G, NA, ACC>(b, n, w, e, f, bad, q, tg);
+                forward_degree_fx<G, NA, ACC>(b, n, w, e, f, bad, p.spad, q, tg);
                 w += ((n + 2) >> 1) * (NA * G);
                 e += n + 1;
                 f = fxs_mul(f, fstep);

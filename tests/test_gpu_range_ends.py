@@ -42,3 +42,32 @@ def test_shifts_next_to_the_z_axis(native, op, dtype, tol):
     got, ref = (run_device(ctx, op, native.PLAIN, src, np.zeros_like(src), p, p, s).astype(np.float64) for s in (sh, axis))
     back = length ** (-deg if op == "m2m" else deg + 1)
     assert rel_err(got * back, ref * back, wo) < tol
+
+
+@pytest.mark.parametrize("op", ("m2l", "l2l"))
+def test_subnormal_sources_keep_their_digits(native, op):
+    """Sources next to the smallest double, raised to normal numbers by the
+    powers of a short (M2L) or long (L2L) shift, give what the same sources
+    2^500 times as large give, bit for bit: only exponents differ.  Elements
+    that are zero have no exponent, so one nonzero element per degree is
+    enough, each in turn."""
+    P, S = 4, 20
+    rng = np.random.default_rng(11)
+    n = 64
+    src = np.zeros((n, S))
+    for i in range(n):
+        # L2L results take the power r^(k - n'): degrees 1 to 3 into normal results of degrees 0 to 2
+        for d in range(1 if op == "l2l" else 0, P):
+            m = rng.integers(0, d + 1)
+            at = [d * (d + 1) + m, (d + 1) ** 2 + m][rng.integers(0, 2 if m else 1)]
+            src[i, at] = np.ldexp(float(rng.integers(1, 64) * 2 + 1), int(rng.integers(-1074, -1060)))
+    u = rng.normal(size=(n, 3))
+    sh = np.ldexp(u / np.linalg.norm(u, axis=1, keepdims=True), -200 if op == "m2l" else 200)
+    p = np.full(n, P, np.uint32)
+    ctx = native.Context(P, "f64")
+    zero = np.zeros((n, S))
+    up = run_device(ctx, op, native.PLAIN, np.ldexp(src, 500), zero, p, p, sh)
+    got = run_device(ctx, op, native.PLAIN, src, zero, p, p, sh)
+    k = slice(0, S if op == "m2l" else 12)
+    assert (np.abs(got[:, k]).max(1) > 0).all()
+    assert np.array_equal(got[:, k], np.ldexp(up, -500)[:, k])
