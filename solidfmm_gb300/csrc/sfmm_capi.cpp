@@ -60,12 +60,10 @@ cudaError_t put(void **dst, const std::vector<T> &v)
 
 }  // namespace
 
-void free_fx(FxDevTables &t)
+void free_arith(ArithTables &t)
 {
-    void *ps[] = {t.W, t.H[0], t.H[1], t.H[2], t.woff, t.hoff};
-    for (void *p : ps)
-        if (p) cudaFree(p);
-    t = FxDevTables{};
+    if (t.mem) cudaFree(t.mem);
+    t = ArithTables{};
 }
 
 void free_tables(DevTables &t)
@@ -88,16 +86,11 @@ void free_offsets(sfmm_context *c)
 
 }  // namespace
 
-// tables of a tensor-core arithmetic, or of FP64 above order 32, once per context
-int ensure_tables(sfmm_context *c, Arith a)
+namespace {
+
+// tables of FP64 above order 32
+int ensure_high(sfmm_context *c)
 {
-    if (is_tc(a)) {
-        const int mode = tc_mode(a);
-        if (c->tc[mode]) return SFMM_OK;
-        cudaError_t e = tc_prepare(&c->tc[mode], mode, c->host);
-        if (e != cudaSuccess) return cuda_fail(c, e, "tensor-core table upload");
-        return SFMM_OK;
-    }
     DevTables &t = c->tab;
     if (t.ready) return SFMM_OK;
     cudaError_t e = put((void **)&c->d_woff, c->host.woff);
@@ -117,70 +110,107 @@ int ensure_tables(sfmm_context *c, Arith a)
     return SFMM_OK;
 }
 
-namespace {
-
-// the tables of one group size: swap coefficients of wsize bytes per woff unit
-template <class T>
-cudaError_t put_fx(FxDevTables &t, const T &h, int P, size_t wsize)
-{
-    cudaError_t e = put(&t.W, h.W);
-    for (int k = 0; k < 3 && e == cudaSuccess; ++k) e = put(&t.H[k], h.H[k]);
-    if (e == cudaSuccess) e = put((void **)&t.woff, h.woff);
-    if (e == cudaSuccess) e = put((void **)&t.hoff, h.hoff);
-    t.wend.assign(P + 1, (int)(h.W.size() * sizeof(h.W[0])));
-    for (int n = 0; n < P; ++n) t.wend[n] = (int)(h.woff[n] * wsize);
-    t.hbytes = (int)(h.H[0].size() * sizeof(h.H[0][0]));
-    t.P = P;
-    return e;
-}
+// arrays laid end to end for one allocation and one copy; add() returns an offset
+struct Blob {
+    std::vector<unsigned char> bytes;
+    template <class T>
+    size_t add(const std::vector<T> &v)
+    {
+        const size_t at = (bytes.size() + 255) & ~size_t(255);
+        bytes.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(&bytes[at], v.data(), v.size() * sizeof(T));
+        return at;
+    }
+};
 
 // edge factors in the arithmetic's form
-cudaError_t put_edges(void **dst, Arith a, const std::vector<double> &e, size_t ne)
+size_t add_edges(Blob &b, Arith a, const std::vector<double> &e, size_t ne)
 {
-    if (a == Arith::F64) return put(dst, fx_edges(e, ne));
+    if (a == Arith::F64) return b.add(fx_edges(e, ne));
     std::vector<float> v;
     for (size_t i = 0; i < ne; ++i) {
         v.push_back((float)e[i]);
         if (a == Arith::FFQ) v.push_back((float)(e[i] - (double)v.back()));
     }
-    return put(dst, v);
+    return b.add(v);
+}
+
+// the tables of one group size: swap coefficients of wsize bytes per woff unit
+template <class T>
+void add_group(Blob &b, FxDevTables &t, size_t (&at)[4], const T &h, int P, size_t wsize)
+{
+    at[0] = b.add(h.W);
+    for (int k = 0; k < 3; ++k) at[1 + k] = b.add(h.H[k]);
+    t.wend.assign(P + 1, (int)(h.W.size() * sizeof(h.W[0])));
+    for (int n = 0; n < P; ++n) t.wend[n] = (int)(h.woff[n] * wsize);
+    t.hbytes = (int)(h.H[0].size() * sizeof(h.H[0][0]));
+    t.P = P;
+}
+
+// tables of the 60-bit fixed-point (F64), the FP32 or the split kernel (FFQ):
+// orders up to 32, both group sizes
+int ensure_fx(sfmm_context *c, Arith a)
+{
+    ArithTables &t = c->fxt[(int)a];
+    if (t.mem) return SFMM_OK;
+    const int P = std::min(c->P, 32);
+    cudaError_t e;
+    try {
+        Blob b;
+        const std::vector<double> *ev[4] = {&c->host.e_in_M, &c->host.e_in_L, &c->host.e_out_L, &c->host.e_out_M};
+        size_t edge[4], at[2][4];
+        for (int k = 0; k < 4; ++k) edge[k] = add_edges(b, a, *ev[k], (size_t)P * (P + 1) / 2);
+        for (int k = 0; k < 2; ++k) {
+            const int G = k ? 8 : 4;
+            if (a == Arith::F32) add_group(b, t.group[k], at[k], build_f32_tables(c->host, G, P), P, sizeof(float));
+            else if (a == Arith::F64) add_group(b, t.group[k], at[k], build_fx_tables(c->host, G, P), P, 2 * sizeof(int32_t));
+            else add_group(b, t.group[k], at[k], build_split_tables(c->host, G, P), P, 2 * sizeof(int32_t));
+        }
+        e = put(&t.mem, b.bytes);
+        const unsigned char *mem = static_cast<const unsigned char *>(t.mem);
+        for (int k = 0; k < 4 && e == cudaSuccess; ++k) t.edge[k] = mem + edge[k];
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+            t.group[k].W = mem + at[k][0];
+            for (int op = 0; op < 3; ++op) t.group[k].H[op] = mem + at[k][1 + op];
+        }
+    } catch (const std::bad_alloc &) {
+        free_arith(t);
+        return fail(c, SFMM_OOM, "operator tables");
+    }
+    if (e != cudaSuccess) {
+        free_arith(t);  // retried from scratch on the next call
+        return cuda_fail(c, e, "table upload");
+    }
+    return SFMM_OK;
 }
 
 }  // namespace
 
-// Tables of the 60-bit fixed-point (F64), the FP32 or the split kernel (FFQ)
-// for G threads per translation (orders up to 32), once per context.
-int ensure_fx(sfmm_context *c, Arith a, int G)
+// Split precision keeps its 1e-7 contract (orthonormal basis) with the
+// fixed-point rotations for M2L and L2L up to order 28 and M2M up to order
+// 18.  Past that the rotation method's own error growth with the degree
+// (about 1.35x per degree for M2M, in every arithmetic) pushes 30-bit
+// mantissas above 1e-7, and the batch runs as SFMM_SPLIT_FF instead.
+constexpr int kFixedM2MOrder = 18;
+
+// Everything that launches of this arithmetic read on this context, whatever
+// their order bound and group size, on its first use: a call of the same
+// arithmetic recorded in a stream capture later allocates nothing.  Split's
+// M2M above kFixedM2MOrder reads the FP64 kernel's tables.
+int ensure_tables(sfmm_context *c, Arith a)
 {
-    FxDevTables &t = c->fxt[(int)a][G == 8];
-    if (t.ready) return SFMM_OK;
-    const int P = std::min(c->P, 32);
-    cudaError_t e = cudaSuccess;
-    try {
-        const std::vector<double> *ev[4] = {&c->host.e_in_M, &c->host.e_in_L, &c->host.e_out_L, &c->host.e_out_M};
-        for (int k = 0; k < 4 && e == cudaSuccess; ++k) {
-            void *&d = c->fx_edge[(int)a][k];
-            if (d) continue;
-            e = put_edges(&d, a, *ev[k], (size_t)P * (P + 1) / 2);
-            if (e != cudaSuccess && d) {
-                cudaFree(d);
-                d = nullptr;
-            }
-        }
-        if (e == cudaSuccess)
-            e = a == Arith::F32   ? put_fx(t, build_f32_tables(c->host, G, P), P, sizeof(float))
-                : a == Arith::F64 ? put_fx(t, build_fx_tables(c->host, G, P), P, 2 * sizeof(int32_t))
-                                  : put_fx(t, build_split_tables(c->host, G, P), P, 2 * sizeof(int32_t));
-    } catch (const std::bad_alloc &) {
-        free_fx(t);
-        return fail(c, SFMM_OOM, "operator tables");
+    if (is_tc(a)) {
+        const int mode = tc_mode(a);
+        if (c->tc[mode]) return SFMM_OK;
+        cudaError_t e = tc_prepare(&c->tc[mode], mode, c->host);
+        if (e != cudaSuccess) return cuda_fail(c, e, "tensor-core table upload");
+        return SFMM_OK;
     }
-    if (e != cudaSuccess) {
-        free_fx(t);  // a partial set is retried from scratch on the next call
-        return cuda_fail(c, e, "table upload");
-    }
-    t.ready = true;
-    return SFMM_OK;
+    if (a == Arith::FF) return SFMM_OK;  // above its orders: no kernel
+    int st = ensure_fx(c, a);
+    if (st == SFMM_OK && a == Arith::FFQ && c->P > kFixedM2MOrder) st = ensure_fx(c, Arith::F64);
+    if (st == SFMM_OK && a == Arith::F64 && c->P > 32) st = ensure_high(c);
+    return st;
 }
 
 int arith_of(sfmm_context *c, int precision, Arith *out)
@@ -204,12 +234,6 @@ int arith_of(sfmm_context *c, int precision, Arith *out)
     return fail(c, SFMM_INVALID_ARG, "unknown precision mode %d", precision);
 }
 
-// Split precision keeps its 1e-7 contract (orthonormal basis) with the
-// fixed-point rotations for M2L and L2L up to order 28 and M2M up to order
-// 18.  Past that the rotation method's own error growth with the degree
-// (about 1.35x per degree for M2M, in every arithmetic) pushes 30-bit
-// mantissas above 1e-7, and the batch runs as SFMM_SPLIT_FF instead.
-constexpr int kFixedM2MOrder = 18;
 // SFMM_SPLIT_FF runs the FP64 kernel, whose 60-bit fixed point needs no more
 // time than float-float did and rounds less: M2L at P=16 86.9 M/s and 3e-15
 // against 80.7 M/s and 7e-14, P=6 605 / 519, P=24 25.2 / 24.0, P=28 14.0 / 14.2.
@@ -223,12 +247,6 @@ Arith resolve_arith(Arith a, int op, int Pbound)
     if (a == Arith::FFQ && op == SFMM_M2M && Pbound > kFixedM2MOrder) a = Arith::FF;
     if (a == Arith::FF && Pbound <= kMaxFloatOrder) a = Arith::F64;
     return a;
-}
-
-// the device tables that a launch of this shape reads (setup_mtx held)
-static int ensure_shape_tables(sfmm_context *c, Arith a, const LaunchShape &s)
-{
-    return s.fx ? ensure_fx(c, a, s.G) : ensure_tables(c, a);
 }
 
 int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *shape)
@@ -257,7 +275,7 @@ int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *sh
     if (shape) *shape = it->second;
     if (it->second.acc == 0)
         return fail(c, SFMM_UNSUPPORTED, "order %d exceeds the GPU kernels' limit %d", Pbound, kMaxKernelOrder);
-    return ensure_shape_tables(c, a, it->second);
+    return ensure_tables(c, a);
 }
 
 void set_shape(sfmm_context *c, std::tuple<int, int, int> key, const LaunchShape *s)
@@ -294,11 +312,7 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
     LaunchShape s;
     int st = prepare_launch(c, op, a, Pbound, &s);
     if (st) return st;
-    if (shape && !is_tc(a)) {
-        s = *shape;
-        std::lock_guard<std::mutex> lk(c->setup_mtx);
-        if ((st = ensure_shape_tables(c, a, s))) return st;
-    }
+    if (shape && !is_tc(a)) s = *shape;
     KParams p{};
     p.op = op;
     p.P = Pbound;
@@ -335,13 +349,11 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
         return SFMM_OK;
     }
     if (s.fx) {
-        const FxDevTables &t = c->fxt[(int)a][s.G == 8];
+        const FxDevTables &t = c->fxt[(int)a].group[s.G == 8];
         p.W = t.W;
-        p.woff = t.woff;
-        p.hoff = t.hoff;
         p.Ptab = t.P;
-        p.ein = c->fx_edge[(int)a][op == SFMM_L2L ? 1 : 0];
-        p.eout = c->fx_edge[(int)a][op == SFMM_M2M ? 3 : 2];
+        p.ein = c->fxt[(int)a].edge[op == SFMM_L2L ? 1 : 0];
+        p.eout = c->fxt[(int)a].edge[op == SFMM_M2M ? 3 : 2];
         p.H = t.H[op];
         p.wbytes = t.wend[Pbound];
         p.hbytes = t.P == Pbound ? t.hbytes : 0;  // a smaller bound reads parts of every row
@@ -575,11 +587,7 @@ void sfmm_destroy(sfmm_context *c)
     cudaSetDevice(c->device);
     free_tables(c->tab);
     for (auto &t : c->tc) tc_release(t);
-    for (auto &ts : c->fxt)
-        for (auto &t : ts) free_fx(t);
-    for (auto &es : c->fx_edge)
-        for (void *p : es)
-            if (p) cudaFree(p);
+    for (auto &t : c->fxt) free_arith(t);
     for (int k = 0; k < 3; ++k) {
         c->d_src[k].release();
         c->d_dst[k].release();
@@ -663,7 +671,7 @@ int sfmm_set_group(sfmm_context *c, int precision, size_t order_bound, int group
     }
     std::lock_guard<std::mutex> lk2(c->setup_mtx);
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
-        if (s[op - SFMM_M2M].fx && (st = ensure_fx(c, resolve_arith(a, op, Pb), s[op - SFMM_M2M].G))) return st;  // before a capture may launch it
+        if ((st = ensure_tables(c, resolve_arith(a, op, Pb)))) return st;  // before a capture may launch it
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
         c->shapes[std::make_tuple(op, (int)resolve_arith(a, op, Pb), Pb)] = s[op - SFMM_M2M];
     return SFMM_OK;

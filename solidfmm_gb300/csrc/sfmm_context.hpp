@@ -30,16 +30,19 @@ struct DevTables {
     bool ready = false;
 };
 
-// device tables of the 60-bit fixed-point, the FP32 or the split kernel
-// (sfmm_tables.hpp, FxTables, F32Tables, SplitTables), one set per group size; the edge factors (e_in_M,
-// e_in_L, e_out_L, e_out_M) are shared by the sets
+// Device tables of the 60-bit fixed-point, the FP32 or the split kernel
+// (sfmm_tables.hpp, FxTables, F32Tables, SplitTables) in one allocation: a set
+// per group size and the edge factors (e_in_M, e_in_L, e_out_L, e_out_M).
 struct FxDevTables {
-    void *W = nullptr, *H[3] = {nullptr, nullptr, nullptr};
-    int *woff = nullptr, *hoff = nullptr;
+    const void *W = nullptr, *H[3] = {nullptr, nullptr, nullptr};
     int P = 0;
     std::vector<int> wend;  // bytes of the swap tables of degrees below an order bound
     int hbytes = 0;         // of one operator's z matrices
-    bool ready = false;
+};
+struct ArithTables {
+    void *mem = nullptr;
+    const void *edge[4] = {};
+    FxDevTables group[2];  // 4 and 8 threads per translation
 };
 
 struct DevBuf {
@@ -94,8 +97,7 @@ struct sfmm_context {
     cudaStream_t stream = nullptr;
     sfmm::HostTables host;
     sfmm::DevTables tab;  // FP64 above order 32
-    sfmm::FxDevTables fxt[sfmm::kNumArith][2];  // by Arith, 4 and 8 threads per translation
-    void *fx_edge[sfmm::kNumArith][4] = {};
+    sfmm::ArithTables fxt[sfmm::kNumArith];  // by Arith
     sfmm::TcDevTables *tc[3] = {nullptr, nullptr, nullptr};  // tensor-core operand images by format
     std::string err;
     std::atomic<uint64_t> launches{0};
@@ -134,7 +136,7 @@ int fail(sfmm_context *c, int st, const char *fmt, ...);
 int cuda_fail(sfmm_context *c, cudaError_t e, const char *what);
 // arithmetic of a precision mode on this context
 int arith_of(sfmm_context *c, int precision, Arith *out);
-// upload the arithmetic's tables once
+// upload the arithmetic's tables once (setup_mtx held)
 int ensure_tables(sfmm_context *c, Arith a);
 // the arithmetic a batch of op with this order bound runs in (split M2M above
 // order 18 runs float-float; tensor-core modes above order 16 run split)

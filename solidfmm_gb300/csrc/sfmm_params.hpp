@@ -46,8 +46,8 @@ struct KParams {
     int atomic;
     int in_hbm;    // expansions in device memory (0: host memory read over the link)
     const void *W;      // arith-typed swap matrices (padded, see sfmm_tables.hpp)
-    const int *woff;    // offset of degree n's W blocks
-    const int *hoff;    // offset of column m's z matrix
+    const int *woff;    // offset of degree n's W blocks (FP64 above order 32)
+    const int *hoff;    // offset of column m's z matrix (FP64 above order 32)
     int rowpad;         // row padding of W and H blocks (8 or 32)
     const void *ein;    // arith-typed forward edge factors (op dependent)
     const void *eout;   // arith-typed backward edge factors (op dependent)
