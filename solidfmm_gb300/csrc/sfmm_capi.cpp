@@ -915,17 +915,12 @@ int sfmm_eval_device(sfmm_context *c, int kind, size_t npts, const double *pos, 
     if (need) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         cudaStreamIsCapturing(c->stream, &cs);
-        const bool grow = cs == cudaStreamCaptureStatusNone;
-        if (gradient && npts >= 4 * nexp) {  // a buffer of its own: other calls' recorded graphs keep theirs
-            const size_t more = eval_scratch_bytes(c->P, (long long)nexp, true);
-            if (grow && c->d_eval_grad.ensure(more) != cudaSuccess) clear_stale_error();
-            pairings = c->d_eval_grad.bytes >= more;
-            if (pairings) scratch = c->d_eval_grad.p;
+        const bool capturing = cs != cudaStreamCaptureStatusNone;
+        if (gradient && npts >= 4 * nexp) {  // a buffer of its own: plain calls need a quarter of it
+            scratch = c->d_eval_grad.take(eval_scratch_bytes(c->P, (long long)nexp, true), capturing);
+            pairings = scratch != nullptr;
         }
-        if (!scratch) {
-            if (grow && c->d_eval.ensure(need) != cudaSuccess) clear_stale_error();
-            if (c->d_eval.bytes >= need) scratch = c->d_eval.p;
-        }
+        if (!scratch) scratch = c->d_eval.take(need, capturing);
     }
     cudaError_t e = launch_eval(c->dtype == SFMM_F64, kind, c->P, (long long)npts, pos, box, E, (long long)stride,
                                 (long long)nexp, centre, potential, gradient, scratch, pairings, c->num_sms, c->stream);

@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <new>
 #include <set>
 #include <tuple>
 #include <string>
@@ -66,6 +67,43 @@ struct DevBuf {
     }
 };
 
+// Scratch that calls recorded in a stream capture may point to: a buffer such
+// a call took stays allocated until the context goes, since its graph may be
+// replayed after the scratch has grown.
+struct GraphBuf {
+    DevBuf buf;
+    bool recorded = false;
+    std::vector<void *> kept;
+    // b bytes, allocated or grown outside captures only; nullptr without them
+    void *take(size_t b, bool capturing)
+    {
+        if (buf.bytes < b) {
+            if (capturing) return nullptr;
+            if (recorded) {
+                try {
+                    kept.push_back(buf.p);
+                } catch (const std::bad_alloc &) {
+                    return nullptr;
+                }
+                buf = DevBuf{};
+                recorded = false;
+            }
+            if (buf.ensure(b) != cudaSuccess) {
+                (void)cudaGetLastError();
+                return nullptr;
+            }
+        }
+        recorded = recorded || capturing;
+        return buf.p;
+    }
+    void release()
+    {
+        buf.release();
+        for (void *p : kept) cudaFree(p);
+        kept.clear();
+    }
+};
+
 struct HostBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -107,8 +145,8 @@ struct sfmm_context {
     int *d_status = nullptr;  // device error word of the translation kernels
     // host-path staging (three pipeline slots for the packed host call)
     sfmm::DevBuf d_src[3], d_dst[3], d_meta[3], d_shift[3], d_work;
-    sfmm::DevBuf d_eval;       // normalised expansions of the float-float L2P/M2P
-    sfmm::DevBuf d_eval_grad;  // the same with the gradient's pairings
+    sfmm::GraphBuf d_eval;       // normalised expansions of the float-float L2P/M2P
+    sfmm::GraphBuf d_eval_grad;  // the same with the gradient's pairings
     sfmm::HostBuf h_src, h_dst, h_meta, h_shift;
     cudaStream_t pipe[3] = {nullptr, nullptr, nullptr};
     // (op, arith, order bound) -> launch shape: operators tuned apart keep
