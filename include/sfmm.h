@@ -284,10 +284,13 @@ int sfmm_bucket_by_order_noalloc(size_t n, const uint32_t *p_in, const uint32_t 
  * float-float on the FP32 pipe over a normalised copy of all nexp
  * expansions, made once per call in context scratch of about
  * nexp * P(P+1) * 8 bytes, four times that with a gradient and four points
- * per expansion or more (allocated or grown on first need; a call inside a stream
- * capture never allocates, and a call without enough scratch runs FP64); error
- * about 1e-14 of the sum of the terms' magnitudes.  Other calls run in FP64.  Calls on one context share the scratch (serialised by a lock,
- * ordered on the context's stream).  Box indices are not range-checked
+ * per expansion or more (allocated or grown on first need, kept until the
+ * context is destroyed; calls without a gradient use the larger buffer where
+ * there is one); error about 1e-14 of the sum of the terms' magnitudes.  A call
+ * inside a stream capture never allocates, and a call without enough scratch
+ * runs FP64; the scratch of a recorded call is not freed when later calls need
+ * more.  Other calls run in FP64.  Calls on one context share the scratch
+ * (serialised by a lock, ordered on the context's stream).  Box indices are not range-checked
  * (device data). */
 int sfmm_eval_device(sfmm_context *ctx, int kind, size_t npts, const double *pos, const uint32_t *box,
                      const void *E, size_t stride, size_t nexp, const double *centre, double *potential,

@@ -74,10 +74,11 @@ struct GraphBuf {
     DevBuf buf;
     bool recorded = false;
     std::vector<void *> kept;
+    bool fits(size_t b) const { return b <= buf.bytes; }
     // b bytes, allocated or grown outside captures only; nullptr without them
     void *take(size_t b, bool capturing)
     {
-        if (buf.bytes < b) {
+        if (!fits(b)) {
             if (capturing) return nullptr;
             if (recorded) {
                 try {

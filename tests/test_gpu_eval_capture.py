@@ -72,3 +72,26 @@ def test_recorded_graph_outlives_growing_scratch(native, gradient):
         got = small.results()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
         del fill
+
+
+@pytest.mark.parametrize("points", [2000, 120])
+def test_gradient_call_sizes_the_scratch_of_recorded_calls(native, points):
+    """After one gradient call with its pairings (four points per expansion),
+    recorded calls without a gradient, and with fewer points, run the same
+    kernels as calls outside a capture: the same bits, not the FP64 kernel's."""
+    import torch
+
+    warm = Batch(2000, 100, 1, True)
+    later = Batch(points, 100, 2, points < 400)
+    outside = native.Context(P, "f64")
+    outside.set_stream(torch.cuda.current_stream().cuda_stream)
+    later.evaluate(outside)
+    want = later.results()
+    ctx = native.Context(P, "f64")
+    ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    warm.evaluate(ctx)
+    warm.results()
+    graph = record(ctx, later)
+    graph.replay()
+    got = later.results()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
