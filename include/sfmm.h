@@ -185,7 +185,8 @@ int sfmm_bounding_sphere(size_t n, const double *x, const double *y, const doubl
 /* Launch shape.  The translation kernels run G threads per translation: 4
  * or 8 for order bounds up to 32, one warp (32) above.  By default a context
  * takes G per (precision, order bound) from a built-in table measured on
- * GB300; sfmm_set_group pins G for one (precision, order bound) pair, and
+ * GB300; sfmm_set_group pins G for one (precision, order bound) pair (FP64
+ * arithmetic above order 16 runs 8 threads where 4 are asked for), and
  * sfmm_tune times every supported G, each with the largest and the smallest
  * tile (translations per CTA) that keep the SM fully occupied, on n synthetic
  * translations of `op` on the context's stream (synchronising it) and keeps

@@ -234,23 +234,29 @@ int arith_of(sfmm_context *c, int precision, Arith *out)
     return fail(c, SFMM_INVALID_ARG, "unknown precision mode %d", precision);
 }
 
+// The tensor-core kernel holds a tile's expansions in tensor memory up to
+// order 16; batches with a larger order bound run the split kernel.
+Arith resolve_mode(Arith a, int op, int Pbound)
+{
+    if (is_tc(a) && Pbound > tc_max_order()) a = Arith::FFQ;
+    if (a == Arith::FFQ && op == SFMM_M2M && Pbound > kFixedM2MOrder) a = Arith::FF;
+    return a;
+}
+
 // SFMM_SPLIT_FF runs the FP64 kernel, whose 60-bit fixed point needs no more
 // time than float-float did and rounds less: M2L at P=16 86.9 M/s and 3e-15
 // against 80.7 M/s and 7e-14, P=6 605 / 519, P=24 25.2 / 24.0, P=28 14.0 / 14.2.
 // Orders above kMaxFloatOrder, which the mode never took, keep Arith::FF and
 // are refused by prepare_launch.
-// The tensor-core kernel holds a tile's expansions in tensor memory up to
-// order 16; batches with a larger order bound run the split kernel.
 Arith resolve_arith(Arith a, int op, int Pbound)
 {
-    if (is_tc(a) && Pbound > tc_max_order()) a = Arith::FFQ;
-    if (a == Arith::FFQ && op == SFMM_M2M && Pbound > kFixedM2MOrder) a = Arith::FF;
-    if (a == Arith::FF && Pbound <= kMaxFloatOrder) a = Arith::F64;
-    return a;
+    a = resolve_mode(a, op, Pbound);
+    return a == Arith::FF && Pbound <= kMaxFloatOrder ? Arith::F64 : a;
 }
 
 int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *shape)
 {
+    const Arith mode = resolve_mode(a, op, Pbound);
     a = resolve_arith(a, op, Pbound);
     if (Pbound < 1) Pbound = 1;
     std::lock_guard<std::mutex> lk(c->setup_mtx);
@@ -269,7 +275,7 @@ int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *sh
     }
     if (a != Arith::F64 && Pbound > kMaxFloatOrder)
         return fail(c, SFMM_UNSUPPORTED, "order %d exceeds %d, the limit of FP32-range arithmetic", Pbound, kMaxFloatOrder);
-    const auto key = std::make_tuple(op, (int)a, Pbound);
+    const auto key = std::make_tuple(op, (int)mode, Pbound);
     auto it = c->shapes.find(key);
     if (it == c->shapes.end()) it = c->shapes.emplace(key, best_shape(a, Pbound, default_group(a, Pbound))).first;
     if (shape) *shape = it->second;
@@ -307,11 +313,11 @@ int run_batch(sfmm_context *c, cudaStream_t stream, int op, Arith a, int Pbound,
     if (n == 0) return SFMM_OK;
     static const char *const kName[3] = {"sfmm m2m launch", "sfmm m2l launch", "sfmm l2l launch"};
     Range range(kName[(op >= SFMM_M2M && op <= SFMM_L2L) ? op - SFMM_M2M : 1]);
-    a = resolve_arith(a, op, Pbound);
-    if (Pbound < 1) Pbound = 1;
     LaunchShape s;
     int st = prepare_launch(c, op, a, Pbound, &s);
     if (st) return st;
+    a = resolve_arith(a, op, Pbound);
+    if (Pbound < 1) Pbound = 1;
     if (shape && !is_tc(a)) s = *shape;
     KParams p{};
     p.op = op;
@@ -673,7 +679,7 @@ int sfmm_set_group(sfmm_context *c, int precision, size_t order_bound, int group
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
         if ((st = ensure_tables(c, resolve_arith(a, op, Pb)))) return st;  // before a capture may launch it
     for (int op = SFMM_M2M; op <= SFMM_L2L; ++op)
-        c->shapes[std::make_tuple(op, (int)resolve_arith(a, op, Pb), Pb)] = s[op - SFMM_M2M];
+        c->shapes[std::make_tuple(op, (int)resolve_mode(a, op, Pb), Pb)] = s[op - SFMM_M2M];
     return SFMM_OK;
 }
 
@@ -726,6 +732,7 @@ int sfmm_tune(sfmm_context *c, int op, int precision, size_t order_bound, size_t
         cleanup();
         return cuda_fail(c, e, "tuning setup");
     }
+    const Arith mode = resolve_mode(a, op, Pb);
     a = resolve_arith(a, op, Pb);
     if (is_tc(a)) {  // one launch shape: time it
         float ms = 0;
@@ -745,7 +752,7 @@ int sfmm_tune(sfmm_context *c, int op, int precision, size_t order_bound, size_t
         if (rate) *rate = ms > 0 ? 3.0 * (double)n / (ms * 1e-3) : 0.0;
         return SFMM_OK;
     }
-    const auto key = std::make_tuple(op, (int)a, Pb);
+    const auto key = std::make_tuple(op, (int)mode, Pb);
     LaunchShape best;
     double best_rate = 0;
     // candidates: every group size that runs at this order, each with the
@@ -768,7 +775,7 @@ int sfmm_tune(sfmm_context *c, int op, int precision, size_t order_bound, size_t
         for (int rep = 0; rep < 2 && st == SFMM_OK; ++rep) {  // warm-up, then timed
             if (rep == 1 && (e = cudaEventRecord(e0, stream)) != cudaSuccess) break;
             for (int k = 0; k < (rep ? 3 : 1) && st == SFMM_OK; ++k)
-                st = run_batch(c, stream, op, a, Pb, (long long)n, src, (long long)S, (long long)n, nullptr, dst,
+                st = run_batch(c, stream, op, mode, Pb, (long long)n, src, (long long)S, (long long)n, nullptr, dst,
                                (long long)S, (long long)n, nullptr, d_ord, d_ord, d_shift, nullptr, 0);
             if (rep == 1 && (e = cudaEventRecord(e1, stream)) != cudaSuccess) break;
         }
@@ -793,7 +800,7 @@ int sfmm_tune(sfmm_context *c, int op, int precision, size_t order_bound, size_t
     set_shape(c, key, &best);
     {
         std::lock_guard<std::mutex> lk2(c->setup_mtx);
-        c->tuned.insert(std::make_tuple(op, (int)a, Pb));
+        c->tuned.insert(std::make_tuple(op, (int)mode, Pb));
     }
     if (group) *group = best.G;
     if (rate) *rate = best_rate;

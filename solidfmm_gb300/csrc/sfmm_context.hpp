@@ -150,13 +150,13 @@ struct sfmm_context {
     sfmm::GraphBuf d_eval_grad;  // the same with the gradient's pairings
     sfmm::HostBuf h_src, h_dst, h_meta, h_shift;
     cudaStream_t pipe[3] = {nullptr, nullptr, nullptr};
-    // (op, arith, order bound) -> launch shape: operators tuned apart keep
+    // (op, mode, order bound) -> launch shape: operators tuned apart keep
     // their own shapes at one order
     std::map<std::tuple<int, int, int>, sfmm::LaunchShape> shapes;
     int *d_woff = nullptr, *d_hoff = nullptr;            // offsets of tab's blocks
     bool pageable_access = false;  // the GPU reads pageable host memory through the host page tables
     sfmm::SlotScratch slot_scratch;  // target table of the classic host call
-    std::set<std::tuple<int, int, int>> tuned;  // (op, arith, order bound) shapes measured by sfmm_tune
+    std::set<std::tuple<int, int, int>> tuned;  // (op, mode, order bound) shapes measured by sfmm_tune
 };
 
 namespace sfmm {
@@ -177,8 +177,11 @@ int cuda_fail(sfmm_context *c, cudaError_t e, const char *what);
 int arith_of(sfmm_context *c, int precision, Arith *out);
 // upload the arithmetic's tables once (setup_mtx held)
 int ensure_tables(sfmm_context *c, Arith a);
-// the arithmetic a batch of op with this order bound runs in (split M2M above
-// order 18 runs float-float; tensor-core modes above order 16 run split)
+// The mode a batch of op with this order bound runs in (split M2M above order
+// 18 runs as split_ff, tensor-core modes above order 16 as split): launch
+// shapes, pinned or measured, belong to it.
+Arith resolve_mode(Arith a, int op, int Pbound);
+// the arithmetic of that mode's kernel (split_ff runs plain FP64's)
 Arith resolve_arith(Arith a, int op, int Pbound);
 // device address of a caller's host array when the kernels can use it
 // directly (pinned host memory, or pageable memory on a GPU that uses the host
@@ -187,7 +190,7 @@ const void *device_view(sfmm_context *c, const void *host);
 // tables and launch shape of (arithmetic, order bound) for op, so that a
 // launch makes no allocation (plans call this before a graph capture)
 int prepare_launch(sfmm_context *c, int op, Arith a, int Pbound, LaunchShape *shape = nullptr);
-// replace (or, with nullptr, drop) the cached launch shape of (op, arith, order bound)
+// replace (or, with nullptr, drop) the cached launch shape of (op, mode, order bound)
 void set_shape(sfmm_context *c, std::tuple<int, int, int> key, const LaunchShape *s);
 // one validated translation launch on device pointers (translation i of the
 // batch is perm[i] when perm is given)

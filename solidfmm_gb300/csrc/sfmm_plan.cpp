@@ -192,7 +192,7 @@ int tune_segment(sfmm_context *c, const sfmm_plan *p, const Stage &s, const Segm
         return SFMM_OK;
     }
     const uint32_t *perm = p->d_perm + s.perm_off + g.off;
-    const auto key = std::make_tuple(s.op, (int)a, g.bound);
+    const auto key = std::make_tuple(s.op, (int)resolve_mode(s.a, s.op, g.bound), g.bound);
     LaunchShape cands[12], best;
     int ncand = 0;
     for (int G : {4, 8, 32})
@@ -231,7 +231,7 @@ int tune_segment(sfmm_context *c, const sfmm_plan *p, const Stage &s, const Segm
     if (e != cudaSuccess) return cuda_fail(c, e, "plan: tuning a segment");
     if (best.acc) {
         std::lock_guard<std::mutex> lk(c->setup_mtx);
-        c->tuned.insert(std::make_tuple(s.op, (int)a, g.bound));
+        c->tuned.insert(key);
         *done = true;
     }
     return SFMM_OK;
@@ -509,7 +509,7 @@ int sfmm_plan_finalize(sfmm_plan *p)
                 if (s.fused) break;  // measured on its own orders above
                 const int bound = s.fused ? s.fused_bound : g.bound;
                 if (is_tc(resolve_arith(s.a, s.op, bound))) continue;  // one shape: nothing to choose
-                const auto key = std::make_tuple(s.op, (int)resolve_arith(s.a, s.op, bound), bound);
+                const auto key = std::make_tuple(s.op, (int)resolve_mode(s.a, s.op, bound), bound);
                 bool have;
                 {
                     std::lock_guard<std::mutex> lk(c->setup_mtx);
