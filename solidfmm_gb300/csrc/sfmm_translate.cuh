@@ -682,16 +682,7 @@ __device__ __forceinline__ void translate_body(const KParams &p)
 #pragma unroll 1
                 for (int s = warp; s < TS; s += nwarps)
                     fx_raise_rows(buf0 + (long long)s * p.spad, p.spad, (int)(m_pin[s] & 0xffffu), lane);
-        // A tile of more than one pair of orders runs all its warps to the
-        // tile's largest: they wait for each other at its end anyway, and in
-        // step they share the instruction cache, which holds a part of the
-        // FP64 kernel's unrolled rows only (translations of random orders in
-        // one launch, M2L: 2 to 10 161 -> 220 M/s, 4 to 16 58 -> 82).
-        bool mixed = false;
-        if constexpr (PL && !F32)
-            mixed = __syncthreads_or(pin != (int)(m_pin[0] & 0xffffu) || pout != (int)m_pout[0]);
-        else
-            __syncthreads();
+        __syncthreads();
 
         // L2 prefetch, spread over the group: this tile's targets (read at the
         // end of the tile) and the next tile's sources (read at its start),
@@ -721,13 +712,24 @@ __device__ __forceinline__ void translate_body(const KParams &p)
         S *b = buf0 + (long long)slot * p.spad;
         int pin_w = __reduce_max_sync(FULL, pin);
         int pout_w = __reduce_max_sync(FULL, pout);
-        if (mixed) {
-            for (int s = lane; s < TS; s += 32) {
-                pin_w = max(pin_w, (int)(m_pin[s] & 0xffffu));
-                pout_w = max(pout_w, (int)m_pout[s]);
+        // A tile of more than one pair of orders runs all its warps to the
+        // tile's largest: they wait for each other at its end anyway, and in
+        // step they share the instruction cache, which holds a part of the
+        // FP64 kernel's unrolled rows only (translations of random orders in
+        // one launch, M2L: 2 to 10 161 -> 220 M/s, 4 to 16 58 -> 82).  Slots
+        // without a translation, and zero shifts, have no orders, and a warp
+        // of them alone does nothing.  Each warp finds this out for itself: a
+        // vote of the CTA at the barrier above cost the registers of a flag
+        // (spills at orders 5 to 24; FMM pass at P=12 36.5 ms, 31.7 now).
+        if constexpr (PL && !F32) {
+            static_assert(kFxThreads / 4 <= 32, "a lane per translation of the tile");
+            const unsigned o = lane < TS ? (m_pin[lane] & 0xffffu) | m_pout[lane] << 16 : 0u;
+            const unsigned some = __ballot_sync(FULL, o != 0u);
+            const unsigned first = __shfl_sync(FULL, o, some ? __ffs(some) - 1 : 0);
+            if ((pin_w | pout_w) && __any_sync(FULL, o != 0u && o != first)) {
+                pin_w = __reduce_max_sync(FULL, o & 0xffffu);
+                pout_w = __reduce_max_sync(FULL, o >> 16);
             }
-            pin_w = __reduce_max_sync(FULL, pin_w);
-            pout_w = __reduce_max_sync(FULL, pout_w);
         }
 
         if constexpr (PL && F32) {
