@@ -405,7 +405,7 @@ LaunchShape translate_shape(Arith a, int P, int G, int ts)
     if (P < 1 || P > kMaxKernelOrder || ts < per_warp || ts % per_warp || G * ts > 256) return s;
     if ((G == 32) != (P > 32)) return s;  // one warp per translation exactly for orders above 32
     int acc = (P + G - 1) / G;
-    if (G == 4) acc = acc <= 2 ? 2 : (acc <= 4 ? 4 : (acc <= 6 ? 6 : 8));
+    if (G == 4) acc = acc <= 2 ? acc : (acc <= 4 ? 4 : (acc <= 6 ? 6 : 8));
     if (G == 32) acc = acc <= 2 ? 2 : 3;
     s.fx = G != 32;
     if (a == Arith::F64 || a == Arith::F32) {
