@@ -284,10 +284,11 @@ int sfmm_bucket_by_order_noalloc(size_t n, const uint32_t *p_in, const uint32_t 
  * Orders up to 32 with at least one point per four expansions run in
  * float-float on the FP32 pipe over a normalised copy of all nexp
  * expansions, made once per call in context scratch of about
- * nexp * P(P+1) * 8 bytes, four times that with a gradient and four points
- * per expansion or more (allocated or grown on first need, kept until the
- * context is destroyed; calls without a gradient use the larger buffer where
- * there is one); error about 1e-14 of the sum of the terms' magnitudes.  A call
+ * nexp * P(P+1) * 8 bytes, four times that with a gradient and eight points
+ * per expansion or more, below order 12 in calls of about 20 000 points or
+ * more only (allocated or grown on first need, kept until the context is
+ * destroyed; calls without a gradient use the larger buffer where there is
+ * one); error about 1e-14 of the sum of the terms' magnitudes.  A call
  * inside a stream capture never allocates, and a call without enough scratch
  * runs FP64; the scratch of a recorded call is not freed when later calls need
  * more.  Other calls run in FP64.  Calls on one context share the scratch

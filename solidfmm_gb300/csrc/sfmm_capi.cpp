@@ -909,12 +909,10 @@ int sfmm_eval_device(sfmm_context *c, int kind, size_t npts, const double *pos, 
     if (!box && nexp < npts) return fail(c, SFMM_INVALID_ARG, "fewer expansions than points without a box index");
     cudaSetDevice(c->device);
     // float-float normalises all nexp expansions into scratch first: worth it
-    // from one point per four expansions on, and with the gradient's pairings
-    // beside each coefficient from four points per expansion on (P=12, 32 points
-    // each: 813 -> 720 us; one point each: level, and slower at low orders).  The scratch is allocated (or grown)
-    // outside stream capture only; a call without enough of it (in a capture,
-    // or when the allocation fails) does without the pairings, or runs the
-    // FP64 kernel.
+    // from one point per four expansions on.  The scratch is allocated (or
+    // grown) outside stream capture only; a call without enough of it (in a
+    // capture, or when the allocation fails) does without the gradient's
+    // pairings, or runs the FP64 kernel.
     std::lock_guard<std::mutex> lk(c->eval_mtx);  // calls share the scratch, in stream order
     void *scratch = nullptr;
     bool pairings = false;
@@ -923,7 +921,7 @@ int sfmm_eval_device(sfmm_context *c, int kind, size_t npts, const double *pos, 
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         cudaStreamIsCapturing(c->stream, &cs);
         const bool capturing = cs != cudaStreamCaptureStatusNone;
-        if (gradient && npts >= 4 * nexp) {  // a buffer of its own: plain calls alone need a quarter of it
+        if (gradient && eval_wants_pairings(c->P, (long long)npts, (long long)nexp, c->num_sms)) {  // a buffer of its own: plain calls alone need a quarter of it
             scratch = c->d_eval_grad.take(eval_scratch_bytes(c->P, (long long)nexp, true), capturing);
             pairings = scratch != nullptr;
         }

@@ -76,6 +76,7 @@ cudaError_t launch_p2x(bool f64, int kind, int P, long long nexp, long long nq, 
 // gradient's pairings or without) for orders up to 32, else (scratch null or
 // higher orders) one FP64 thread per point.
 size_t eval_scratch_bytes(int P, long long nexp, bool pairings);
+bool eval_wants_pairings(int P, long long npts, long long nexp, int num_sms);
 cudaError_t launch_eval(bool f64, int kind, int P, long long npts, const double *pos, const uint32_t *box,
                         const void *E, long long stride, long long nexp, const double *centre, double *pot,
                         double *grad, void *scratch, bool pairings, int num_sms, cudaStream_t st);

@@ -785,8 +785,7 @@ struct ff_scale {
     __device__ __forceinline__ ff operator()(ff v) const { return ff{__fmul_rn(__fmul_rn(v.hi, f1), f2), __fmul_rn(__fmul_rn(v.lo, f1), f2)}; }
 };
 // How a point's gradient is formed: not at all, from the prepared pairings
-// (half the work per point, 110 more operations per coefficient of every
-// expansion: from four points per expansion on), or from e itself.
+// (half the work per point, eval_wants_pairings), or from e itself.
 enum { GRAD_NONE = 0, GRAD_PREPARED = 1, GRAD_DIRECT = 2 };
 
 // C lanes per point, the columns m dealt to them back and forth (their
@@ -922,6 +921,24 @@ __global__ void __launch_bounds__(128, GRAD == GRAD_PREPARED && C == 1 ? 6 : 1) 
     }
 }
 
+// Few points: four lanes each.  The lines are where the sides meet on 152 SMs
+// (potential, one lane against four: P=4 10 000 points 14.0 us / 13.9, 30 000
+// 14.6 / 18.1; P=12 20 000 39 / 30, 30 000 41 / 41; P=24 38 000 128 / 117;
+// below order 4 four never win by more than a launch's jitter).
+static bool eval_few(int P, long long npts, int num_sms)
+{
+    return P >= 4 && npts < (long long)num_sms * (P < 16 ? 128 : 256);
+}
+// Pairings cost 110 operations per coefficient of every expansion, by as many
+// threads as there are degrees: worth it from eight points per expansion on
+// (prepared against direct at 200 000 points: four each 1.04 to 1.16 times the
+// time, eight 0.93 to 1.02, 32 0.83 to 0.89), but not for few points of low
+// order (P=4, 3 000 points 15.3 against 13.4 us; P=16, 10 000 50 against 57).
+bool eval_wants_pairings(int P, long long npts, long long nexp, int num_sms)
+{
+    return npts >= 8 * nexp && (P >= 12 || npts >= (long long)num_sms * 128);
+}
+
 // scratch of the normalised copy, with or without the gradient's pairings
 size_t eval_scratch_bytes(int P, long long nexp, bool pairings)
 {
@@ -980,7 +997,7 @@ cudaError_t launch_eval(bool f64, int kind, int P, long long npts, const double 
         if (f64) eval_prep<double>(kind, P, nexp, E, stride, Mn, sdeg, pairings, st);
         else eval_prep<float>(kind, P, nexp, E, stride, Mn, sdeg, pairings, st);
         const EvalArgs a{kind, P, npts, pos, box, Mn, sdeg, centre, pot, grad};
-        const bool few = npts < (long long)num_sms * 256;
+        const bool few = eval_few(P, npts, num_sms);
         if (!grad || kind != 0) eval_points<GRAD_NONE>(a, few, st);
         else if (pairings) eval_points<GRAD_PREPARED>(a, few, st);
         else eval_points<GRAD_DIRECT>(a, few, st);

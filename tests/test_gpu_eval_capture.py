@@ -64,7 +64,7 @@ def test_recorded_graph_outlives_growing_scratch(native, gradient):
     want = small.results()
     graph = record(ctx, small)
     for nexp in (500, 5000):
-        for later in (Batch(4 * nexp, nexp, nexp, True), Batch(nexp, nexp, nexp + 1, False)):
+        for later in (Batch(16 * nexp, nexp, nexp, True), Batch(nexp, nexp, nexp + 1, False)):
             later.evaluate(ctx)
             later.results()
         fill = torch.full((1 << 20,), float("nan"), device="cuda:0")  # what memory given back may come to hold
@@ -76,7 +76,7 @@ def test_recorded_graph_outlives_growing_scratch(native, gradient):
 
 @pytest.mark.parametrize("points", [2000, 120])
 def test_gradient_call_sizes_the_scratch_of_recorded_calls(native, points):
-    """After one gradient call with its pairings (four points per expansion),
+    """After one gradient call with its pairings (20 points per expansion),
     recorded calls without a gradient, and with fewer points, run the same
     kernels as calls outside a capture: the same bits, not the FP64 kernel's."""
     import torch
