@@ -543,19 +543,12 @@ __global__ void __launch_bounds__(kTcRows *NWG, 1) k_translate_tc(KParams p, TcT
         // float-float (FP32 and integer pipes; the FP64 pipe runs at 1/64 of
         // the FP32 rate), this thread's orders m in [j0, j0 + LPT), stored as FP32
         {
-            const ff fx = ff_from_d_int(x), fy = ff_from_d_int(y), fz = ff_from_d_int(z);
-            const ff rxy2 = A::dot2(fx, fx, fy, fy);
-            const ff rxy = ff_sqrt(rxy2);
-            const ff rr = ff_sqrt(A::add(rxy2, A::mul(fz, fz)));
+            const ff fz = ff_from_d_int(z);
+            const ff_transverse tr = ff_transverse_of(x, y);
+            const ff rr = ff_sqrt(A::add(tr.r2, A::mul(fz, fz)));
             const ff ri = ff_rcp(rr), one{1.f, 0.f}, zero{0.f, 0.f};
-            ff e1c = one, e1s = zero;
-            if (rxy.hi > 0.f) {
-                const ff rq = ff_rcp(rxy);
-                e1c = A::mul(fy, rq);
-                e1s = A::mul(fx, rq);
-            }
-            const ff b1c = A::mul(fz, ri), b1s = A::neg(A::mul(rxy, ri));
-            ff eac = e1c, eas = e1s, ebc = b1c, ebs = b1s;
+            const ff b1c = A::mul(fz, ri), b1s = A::neg(A::mul(tr.r, ri));
+            ff eac = tr.c, eas = tr.s, ebc = b1c, ebs = b1s;
             // forward scale r^n (local input) or r^-(n+1) (multipole input);
             // backward r^(n+1) (multipole output) or r^-n (local output)
             ff f = op == OP_L2L ? one : ri, g = op == OP_M2M ? rr : one;
@@ -595,7 +588,7 @@ __global__ void __launch_bounds__(kTcRows *NWG, 1) k_translate_tc(KParams p, TcT
                     if (m < max(pin, pout) && !(isfinite(f.hi) && isfinite(g.hi) && f.hi != 0.f && g.hi != 0.f))
                         range_ok = false;
                 }
-                tcd::cmul_ff(ac, as, e1c, e1s);
+                tcd::cmul_ff(ac, as, tr.c, tr.s);
                 tcd::cmul_ff(bc, bs, b1c, b1s);
                 f = A::mul(f, f1);
                 g = A::mul(g, g1);

@@ -448,17 +448,12 @@ struct SplitGeometry {
     __device__ __forceinline__ SplitGeometry(double x, double y, double z, int q)
     {
         using A = arith<ff>;
-        const ff fx = ff_from_d_int(x), fy = ff_from_d_int(y), fz = ff_from_d_int(z);
-        const ff rxy2 = A::dot2(fx, fx, fy, fy);
-        const ff rxy = ff_sqrt(rxy2);
-        r = ff_sqrt(A::add(rxy2, A::mul(fz, fz)));
+        const ff fz = ff_from_d_int(z);
+        const ff_transverse t = ff_transverse_of(x, y);
+        r = ff_sqrt(A::add(t.r2, A::mul(fz, fz)));
         rinv = ff_rcp(r);
-        cff ea{ff{1.f, 0.f}, ff{0.f, 0.f}};
-        if (rxy.hi > 0.f) {
-            const ff rr = ff_rcp(rxy);
-            ea = cff{A::mul(fy, rr), A::mul(fx, rr)};
-        }
-        const cff eb{A::mul(fz, rinv), A::neg(A::mul(rxy, rinv))};
+        const cff ea{t.c, t.s};
+        const cff eb{A::mul(fz, rinv), A::neg(A::mul(t.r, rinv))};
         auto cm = [](cff a, cff b) {
             return cff{A::dot2(a.c, b.c, A::neg(a.s), b.s), A::dot2(a.s, b.c, a.c, b.s)};
         };
