@@ -73,6 +73,39 @@ def z_flops(op, P):
     return sum(2 * (P - m) * (P - m + 1) for m in range(P))
 
 
+# what the printed line keeps of the headline run: it has to stay short enough
+# for a log's tail (under 2 000 characters); the whole record, notes and the
+# other workloads' rows among it, goes to standard error
+SUMMARY = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+           "vs_baseline", "dtype", "data", "config", "e2e", "roofline", "plain_fp64", "split_over_plain_fp64",
+           "tensor_core", "cpu_baseline", "clocks", "gpu_launches")
+
+
+def summary(line):
+    def short(v):
+        if isinstance(v, float):
+            return float(f"{v:.6g}")
+        if isinstance(v, dict):
+            return {k: short(x) for k, x in v.items()}
+        return [short(x) for x in v] if isinstance(v, (list, tuple)) else v
+
+    out = {k: line[k] for k in SUMMARY if k in line}
+    for k, keep in (("roofline", ("bound", "achieved", "peak", "unit", "frac", "traffic", "peak_source", "kernel")),
+                    ("e2e", ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")),
+                    ("cpu_baseline", ("value", "unit", "cores", "kind")),
+                    ("clocks", ("sm_mhz", "sm_max_mhz", "reasons"))):
+        if out.get(k):
+            out[k] = {x: out[k][x] for x in keep if x in out[k]}
+    if out.get("tensor_core"):
+        out["tensor_core"] = {name: row["value"] for name, row in out["tensor_core"].items()}
+    acc = line.get("accuracy_vs_fp64_oracle_1000") or {}
+    out["error_vs_fp64_oracle"] = {k: v for k, v in acc.items() if isinstance(v, float)}
+    out = short(out)
+    for k in ("value", "ms_per_step"):  # in full
+        out[k] = line[k]
+    return out
+
+
 def useful_flops(op, P):
     """Algorithmic flops of one translation (rotations + z-translation), equal orders."""
     rot = 2 * sum(4 * d * d + 16 * d for d in range(1, P + 1))
@@ -1012,7 +1045,7 @@ def main():
             "unit": "GB/s", "frac": t_roof / t_kernel, "traffic": tb * N if tb else None,
             "traffic_source": (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of the split kernel, "
                                f"{tb:.0f} B per translation on 65 536 translations, scaled to {N}") if tb else None,
-            "peak_source": peak_src, "kernel": "k_translate<ff, G, ACC, fixed, in HBM> (split)",
+            "peak_source": peak_src, "kernel": "k_translate_split",
             "bytes_per_translation": B, "useful_flops_per_translation": F,
             "t_roof_ns_per_translation": {"hbm": t_hbm * 1e9, "fp32_pipe": t_fp32 * 1e9, "fp64_pipe": 0.0,
                                           "tensor_pipe": 0.0},
@@ -1102,7 +1135,8 @@ def main():
         del src, dst, h_src, h_dst
         torch.cuda.empty_cache()
         line["configs"] = extras(args, local)
-    print(json.dumps(line))
+    print(json.dumps(line), file=sys.stderr)
+    print(json.dumps(summary(line)))
 
 
 if __name__ == "__main__":
