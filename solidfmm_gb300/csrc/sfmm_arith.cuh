@@ -47,27 +47,15 @@ struct arith<double> {
     static __device__ __forceinline__ T dot2(T a1, T b1, T a2, T b2) { return fma(a1, b1, a2 * b2); }
 };
 
+// what the FP32 kernel's gather and target update use (its stages: sfmm_f32.cuh)
 template <>
 struct arith<float> {
     static constexpr bool split = false;
     using T = float;
     using Stor = float;
-    using Acc = float;
     static __device__ __forceinline__ T zero() { return 0.f; }
-    static __device__ __forceinline__ T from_d(double x) { return (float)x; }
-    static __device__ __forceinline__ T from_src(float x) { return x; }
-    static __device__ __forceinline__ double to_d(T x) { return (double)x; }
-    static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
-    static __device__ __forceinline__ T add(T a, T b) { return a + b; }
-    static __device__ __forceinline__ T sub(T a, T b) { return a - b; }
-    static __device__ __forceinline__ T neg(T a) { return -a; }
-    static __device__ __forceinline__ Acc acc0() { return 0.f; }
-    static __device__ __forceinline__ void mac(Acc &acc, T w, T x) { acc = fmaf(w, x, acc); }
-    static __device__ __forceinline__ T fin(Acc a) { return a; }
     static __device__ __forceinline__ T ld(const Stor *p) { return *p; }
     static __device__ __forceinline__ void st(Stor *p, T v) { *p = v; }
-    static __device__ __forceinline__ T ldt(const T *p) { return __ldg(p); }
-    static __device__ __forceinline__ T dot2(T a1, T b1, T a2, T b2) { return fmaf(a1, b1, a2 * b2); }
 };
 
 // Fast2Sum: |a| >= |b| assumed (or a == 0)

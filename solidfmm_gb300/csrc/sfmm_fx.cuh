@@ -268,9 +268,7 @@ __device__ __forceinline__ void fx_powers(long long c1, long long s1, int r, int
 // applied to the mantissas of the lane's part.  The coefficients of column
 // slot t (column j0 + 2t, j0 = (r + n + part) & 1) lie together, lane by
 // lane: NA/2 int4 per lane for pairs of rows, then an int2 for an odd last
-// one, so a lane fetches two rows by one 16-byte load.  A degree of NA blocks
-// has NA RS/2 slots or one less, so the loop is unrolled completely and every
-// address is an immediate offset.
+// one, so a lane fetches two rows by one 16-byte load.
 template <int G, int NA>
 __device__ __forceinline__ void swap_fx(const int2 *__restrict__ W, const double *own, int j0, int cnt, int q,
                                         long long round, long long (&out)[NA])

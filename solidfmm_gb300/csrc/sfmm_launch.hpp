@@ -50,7 +50,7 @@ int default_group(Arith a, int P);
 // CTAs of at least min_threads threads when one fits
 LaunchShape best_shape(Arith a, int P, int G, bool small_tiles = false, int min_threads = 128);
 
-// Launch the fused translation kernel (defined in sfmm_k{64,32,ff,ffq}.cu).
+// Launch the fused translation kernel (defined in sfmm_k{64,fx,32,ffq}.cu).
 cudaError_t launch_translate(Arith a, const KParams &p, const LaunchShape &s, int grid, cudaStream_t st);
 int translate_blocks_per_sm(Arith a, const LaunchShape &s);
 

@@ -55,7 +55,6 @@ struct KParams {
     int wbytes, hbytes; // 60-bit kernel: bytes of W and H that this order bound reads
     int spad;           // buffer elements per translation
     int TS;             // translations per CTA tile
-    void *scratch;      // global buffer (GBUF kernels)
     int *status;        // device error word: bit 0 = a translation had an out-of-range index or order
     // pointer mode (both null otherwise): translation t reads its source at
     // src_ptr[t] and accumulates into dst_ptr[t] (addresses the GPU can use,

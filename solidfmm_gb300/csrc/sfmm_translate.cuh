@@ -409,9 +409,6 @@ __device__ __forceinline__ int degree_at(int c) { return (int)__ldg(kDegree.d + 
 // source coefficient times 2^e in the arithmetic's storage type (exact)
 __device__ __forceinline__ ff src_scaled(double x, int e, const ff *) { return ff_from_d_scaled0(x, e); }
 __device__ __forceinline__ float src_scaled(float x, int e, const float *) { return f_scaled(x, e); }
-// FP64 sources of the FP32 kernel: scaled in FP64 first, so that sources
-// beyond the FP32 range come into it
-__device__ __forceinline__ float src_scaled(double x, int e, const float *) { return (float)d_scaled(x, e); }
 
 // Per-thread geometry of one translation in FP64 (orders above 32): |shift|,
 // its inverse and the rotation factors.
