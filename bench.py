@@ -99,7 +99,7 @@ def summary(line):
     if out.get("tensor_core"):
         out["tensor_core"] = {name: row["value"] for name, row in out["tensor_core"].items()}
     acc = line.get("accuracy_vs_fp64_oracle_1000") or {}
-    out["error_vs_fp64_oracle"] = {k: v for k, v in acc.items() if isinstance(v, float)}
+    out["error_vs_fp64_oracle"] = {k: v["rel_l2_orthonormal_max"] for k, v in acc.items() if isinstance(v, dict)}
     out = short(out)
     for k in ("value", "ms_per_step"):  # in full
         out[k] = line[k]

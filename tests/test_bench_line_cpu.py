@@ -22,7 +22,8 @@ def test_printed_line_is_short_and_complete():
             "config": {"workload": "w" * 200, "global_batch": 2000000, "parallelism": "replica1", "l2": "l" * 60},
             "plain_fp64": {"value": v, "ms_per_step": v}, "split_over_plain_fp64": 1.1578901234,
             "split_ff": {"value": v, "ms_per_step": v, "note": long},
-            "accuracy_vs_fp64_oracle_1000": {"split": 3.6e-9, "plain_fp64": 3.6e-15, "metric": long, "per_degree": [v] * 16},
+            "accuracy_vs_fp64_oracle_1000": {k: {"rel_l2_orthonormal_max": 3.6364e-9, "per_degree": [v] * 16}
+                                             for k in ("plain_fp64", "split", "split_ff", "tc_tf32x3", "tc_bf16x3", "tc_bf16x6")},
             "physics_checks": {"what": long, "rows": [{"a": v}] * 30},
             "e2e": {"value": v, "unit": "translations/s", "h2d_bytes_per_step": 4688000000,
                     "d2h_bytes_per_step": 4352000000, "api": long},
@@ -39,4 +40,5 @@ def test_printed_line_is_short_and_complete():
         assert k in out, k
     assert out["value"] == v and out["ms_per_step"] == line["ms_per_step"]
     assert out["e2e"]["h2d_bytes_per_step"] == 4688000000 and out["e2e"]["d2h_bytes_per_step"] == 4352000000
+    assert out["error_vs_fp64_oracle"]["split"] == 3.6364e-9
     assert out["clocks"] == line["clocks"] and out["config"] == line["config"]
