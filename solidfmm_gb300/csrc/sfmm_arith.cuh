@@ -320,7 +320,7 @@ struct arith<ff> {
 };
 
 // The transverse part (x, y) of a shift in float-float: its length, the square
-// of that, and (c, s) = (y, x) / length, (1, 0) for none.  Below 2^-30 beside a
+// of that, and (c, s) = (y, x) / length, (1, 0) for none.  Below 2^-29 beside a
 // shift of length 2 to 7 the components take a power of two of their own:
 // their squares' low words, then the squares, leave the FP32 range there, and
 // (c, s) would lose unit length, while the square adds nothing to |shift|^2.
@@ -330,10 +330,17 @@ struct ff_transverse {
 __device__ __forceinline__ ff_transverse ff_transverse_of(double x, double y)
 {
     using A = arith<ff>;
-    const int k = max(exp_of(x), exp_of(y)), up = k < -30 ? -k : 0;
-    const ff fx = ff_from_d_scaled0(x, up), fy = ff_from_d_scaled0(y, up);
+    ff fx = ff_from_d_int(x), fy = ff_from_d_int(y);
     ff_transverse t;
     t.r2 = A::dot2(fx, fx, fy, fy);
+    int down = 0;
+    if (t.r2.hi < 0x1p-58f) {
+        const int k = max(exp_of(x), exp_of(y));
+        fx = ff_from_d_scaled0(x, -k);
+        fy = ff_from_d_scaled0(y, -k);
+        down = max(k, -252);
+        t.r2 = A::dot2(fx, fx, fy, fy);
+    }
     t.r = ff_sqrt(t.r2);
     t.c = ff{1.f, 0.f};
     t.s = ff{0.f, 0.f};
@@ -342,9 +349,8 @@ __device__ __forceinline__ ff_transverse ff_transverse_of(double x, double y)
         t.c = A::mul(fy, ri);
         t.s = A::mul(fx, ri);
     }
-    if (up) {
-        const int e = max(-up, -252);
-        t.r = ff{ldexp2(t.r.hi, e), ldexp2(t.r.lo, e)};
+    if (down) {
+        t.r = ff{ldexp2(t.r.hi, down), ldexp2(t.r.lo, down)};
         t.r2 = ff{0.f, 0.f};
     }
     return t;

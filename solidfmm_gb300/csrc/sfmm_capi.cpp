@@ -243,9 +243,13 @@ Arith resolve_mode(Arith a, int op, int Pbound)
     return a;
 }
 
-// SFMM_SPLIT_FF runs the FP64 kernel, whose 60-bit fixed point needs no more
-// time than float-float did and rounds less: M2L at P=16 86.9 M/s and 3e-15
-// against 80.7 M/s and 7e-14, P=6 605 / 519, P=24 25.2 / 24.0, P=28 14.0 / 14.2.
+// SFMM_SPLIT_FF runs the FP64 kernel, whose 60-bit fixed point rounds less than
+// float-float did (M2L P=16 2e-15 against 7e-14) and is as fast or faster but for
+// some batches: M2L in M/s, fixed point / float-float, P=6 592 / 499, P=16 86.5 /
+// 77.8, P=20 47.7 / 44.8, P=22 30.9 / 33.2, P=24 22.1 / 23.5, P=26 15.6 / 17.9,
+// P=28 13.5 / 13.5; FMM pass at P=12 31.5 / 35.4 ms; one translation at P=12 68 /
+// 56 us; orders 4 to 24 in no order 20.5 / 27.5 (plans sort them).  No shape of
+// the fixed-point kernel closes those, and its accuracy is what the mode has now.
 // Orders above kMaxFloatOrder, which the mode never took, keep Arith::FF and
 // are refused by prepare_launch.
 Arith resolve_arith(Arith a, int op, int Pbound)
@@ -477,12 +481,12 @@ LaunchShape best_shape(Arith a, int P, int G, bool small_tiles, int min_threads)
     // a lower L1 hit rate for the tables); smaller CTAs when no larger tile
     // fits, or when sfmm_tune measures them faster (split P=27: +6%).  The
     // 60-bit kernel also takes two warps (three above order 22) where they
-    // hold an eighth more threads: M2L P=21 33.2 -> 37.7 M/s, P=24 20.4 ->
-    // 22.3, P=30 8.3 -> 11.1, while with fewer (P=20) or equal numbers four win
-    // (47.7 against 42.0).  One- and two-warp CTAs would give P=24 25.3 and
-    // 24.0, but only while all of them run in step: on a launch of orders 4 to
-    // 24 in no order they wait for instructions (9.1 and 14.7 M/s; three warps
-    // 20.3, four 22.5), which up to order 22 costs nothing (32.5 against 32.4).
+    // hold an eighth more threads: M2L P=21 1.72 ms (2.01 with four warps), P=24
+    // 2.01 (2.18), P=30 2.22 (2.82), while with equal numbers they are level
+    // (P=22, 23, 26) or four win (P=20 1.60, two 1.77).  One- and two-warp CTAs
+    // would give P=24 1.77 and 1.85, but only while all of them run in step: a
+    // launch of orders 4 to 24 in no order, whose warps wait for instructions,
+    // takes 4.30 and 2.78 ms with them, 2.17 with three and 2.00 with four.
     const int few = a == Arith::F64 ? (P <= 22 ? 64 : 96) : 32;
     LaunchShape best[2];
     long most[2] = {0, 0};

@@ -20,8 +20,8 @@
 // scheduler, an integer 32x32+64-bit one for four: three of them per term leave
 // the FP64 pipe to the z-translation, whose coefficients span too many orders of
 // magnitude for a block exponent, and to the accumulation into the targets.
-// Measured (M2L, one GB300): P=16 37.1 -> 86.9 M/s, P=8 168 -> 387, P=24 11.7
-// -> 25.2, with an error no larger than the FP64 transforms' (P=16 M2L 2.1e-15
+// Measured (M2L, one GB300): P=16 37.1 -> 86.2 M/s, P=8 168 -> 387, P=24 11.7
+// -> 22.1, with an error no larger than the FP64 transforms' (P=16 M2L 2.1e-15
 // against 3.4e-15, M2M 7.1e-17 against 9.1e-17, P=21 L2L 2e-16 against 4.5e-15).
 // What bounds it now: the FP64 pipe is busy 55% of
 // the time with the z-translation alone, the schedulers issue in 45% of the

@@ -1025,12 +1025,12 @@ __global__ void __launch_bounds__(kFxThreads, fx_blocks<A>(ACC)) k_translate_fx(
 }
 
 // Resident CTAs per SM that the registers have to allow.  Four threads per
-// translation: four CTAs at orders up to 4 (P=2 314 us, 327 with three), three
-// at 5 to 8 (four spill: orders 2 to 6 in one launch 688 us, 624 with three),
-// two at 9 to 16 (P=12 206 M/s, 166 with three).  Eight threads at orders 25 to
-// 28: not more registers than twelve warps leave each other (168; with 174
-// only eight of the ten that shared memory allows were resident, P=25 1.83 ms,
-// 1.54 so).
+// translation: four CTAs at orders up to 4 (P=2 291 us, 327 with three), three
+// at 5 to 8 (four spill 148 bytes: orders 2 to 6 in one launch 688 us, 621 with
+// three, whose 16 bytes lie outside the stages), two at 9 to 16 (P=12 206 M/s,
+// 166 with three).  Eight threads at orders 25 to 28: not more registers than
+// twelve warps leave each other (168; with 179 only eight of the ten that shared
+// memory allows were resident, P=25 1.83 ms, 1.55 so).
 constexpr int split_blocks(int G, int acc)
 {
     return G == 4 ? (acc <= 1 ? 4 : acc <= 2 ? 3 : acc <= 4 ? 2 : 1) : acc <= 2 ? 3 : acc == 3 ? 2 : 1;
