@@ -59,7 +59,8 @@ typedef enum { SFMM_M2M = 0, SFMM_M2L = 1, SFMM_L2L = 2 } sfmm_op;
  *           arithmetic: there the rotation method's error growth with the
  *           degree would take 30-bit mantissas past 1e-7.
  * SPLIT_FF: FP64's own accuracy for the whole translation (orders <= 28);
- *           runs the PLAIN kernel of an SFMM_F64 context.
+ *           runs the PLAIN kernel of an SFMM_F64 context, with launch shapes
+ *           of its own.
  * TC_TF32:  the tensor-core kernel (tcgen05, one thread per translation,
  *           128 translations per MMA tile): every swap and z-translation is
  *           an MMA against constant matrices held in shared memory, with both
@@ -130,7 +131,10 @@ int sfmm_set_stream(sfmm_context *ctx, void *stream);
  * Shifts are FP64 for both data types.  Asynchronous on the context's stream.
  * Entries with an index or order out of range are skipped and flagged in the
  * context's device status word (sfmm_device_status); they never touch memory
- * out of bounds.  Targets must not alias sources. */
+ * out of bounds.  Targets must not alias sources.  The first call of a
+ * precision mode on a context uploads its operator tables; later calls of the
+ * mode, at any order bound, allocate nothing and may be recorded in a stream
+ * capture. */
 int sfmm_translate_device(sfmm_context *ctx, int op, int precision, size_t n,
                           const void *src, size_t src_stride, size_t src_count, const uint32_t *src_index,
                           void *dst, size_t dst_stride, size_t dst_count, const uint32_t *dst_index,
